@@ -233,73 +233,110 @@ __host__ __device__ inline float f32_from(uint32_t b) {
 #endif
 }
 
-// m <= kFastMantissaF64.
+// The signed forms below fold the sign into the linear region's rounding
+// constant (1.5 * 2^52, 1.5 * 2^23: rint is symmetric, so rint(x 2^L) is
+// +-rint(|x| 2^L) and its two's complement appears in the low word / bits),
+// and the log region's two additions into one constant: 9 instead of 13
+// instructions a component to quantise, 7 instead of 11 to dequantise.
+//
+// m <= kFastMantissaF64.  The log region needs no clamp: its shift is at
+// least 1, so the code is at most (2^31 - 1) >> 1 = kCodeLimit.
 __host__ __device__ inline int32_t quantize_fast(double x, CodecParams p) {
     const uint32_t hi = hi_word(x), ahi = hi & 0x7fffffffu;
     const int e0 = p.m - p.L;
     const uint32_t thr = uint32_t(e0 + 1023) << 20;
-    // linear region: rint(|x| 2^L) appears in the low word of fma(|x|, 2^L, 2^52)
-    const double a = from_words(ahi, lo_word(x));
     const double scale = from_words(uint32_t(p.L + 1023) << 20, 0u);
 #ifdef __CUDA_ARCH__
-    const double r = __fma_rn(a, scale, 4503599627370496.0);
+    const double r = __fma_rn(x, scale, 6755399441055744.0);
 #else
-    const double r = std::fma(a, scale, 4503599627370496.0);
+    const double r = std::fma(x, scale, 6755399441055744.0);
 #endif
-    const uint32_t c_lin = lo_word(r);
     // log region: round the high word to m mantissa bits (the rounding bit is
-    // bit 19 - m of the high word)
+    // bit 19 - m of the high word), minus (e0 + 1023 - 1) 2^m
     const int shh = 20 - p.m;
-    const uint32_t c_log = ((ahi + (1u << (shh - 1))) >> shh) - (uint32_t(e0 + 1023) << p.m) + (1u << p.m);
-    uint32_t c = ahi < thr ? c_lin : c_log;
-    if (ahi >= thr && c > (uint32_t)kCodeLimit) c = (uint32_t)kCodeLimit;
+    const uint32_t c_log = (ahi + ((1u << (shh - 1)) + (1u << 20) - thr)) >> shh;
     const uint32_t sgn = (uint32_t)((int32_t)hi >> 31);
-    return (int32_t)((c ^ sgn) - sgn);
+    return ahi < thr ? (int32_t)lo_word(r) : (int32_t)((c_log ^ sgn) - sgn);
+}
+
+// A code of the linear region (|q| <= 2^m): q in the low word of
+// 2^(52-L) (1 + (2^31 + q) 2^-52), minus 2^(52-L) (1 + 2^-21).
+__host__ __device__ inline double dequantize_linear(int32_t q, CodecParams p, double) {
+    const uint32_t ehi = uint32_t(1075 - p.L) << 20;
+    return from_words(ehi, (uint32_t)q ^ 0x80000000u) - from_words(ehi, 0x80000000u);
 }
 
 // m <= kFastMantissaF64.
 __host__ __device__ inline double dequantize_fast(int32_t q, CodecParams p) {
-    const uint32_t sgn = (uint32_t)(q >> 31);
-    const uint32_t c = ((uint32_t)q ^ sgn) - sgn;
-    // linear region: c in the low word of 2^(52-L) (1 + c 2^-52), minus 2^(52-L)
-    const uint32_t ehi = uint32_t(1075 - p.L) << 20;
-    const double lin = from_words(ehi, c) - from_words(ehi, 0u);
-    // log region: the code is the high word of the value, shifted
+    const double lin = dequantize_linear(q, p, 0.0);
+    // log region: the code's magnitude is the high word of the value, shifted
+    const uint32_t c = (uint32_t)(q < 0 ? -q : q);
     const int e0 = p.m - p.L;
-    const uint32_t lhi = (c + (uint32_t(e0 + 1023) << p.m) - (1u << p.m)) << (20 - p.m);
-    const double a = c <= (1u << p.m) ? lin : from_words(lhi, 0u);
-    return from_words(hi_word(a) | (sgn & 0x80000000u), lo_word(a));
+    const uint32_t lhi = (c << (20 - p.m)) + (uint32_t(e0 + 1022) << 20);
+    return c <= (1u << p.m) ? lin : from_words(lhi | ((uint32_t)q & 0x80000000u), 0u);
 }
+
+// Largest m of the signed linear form in single precision: |q| <= 2^22 keeps
+// 1.5 * 2^23 + q inside the binade whose spacing is 1.
+constexpr int kSignedMantissaF32 = 22;
 
 __host__ __device__ inline int32_t quantize_fast(float x, CodecParams p) {
     const uint32_t bits = f32_bits(x), abits = bits & 0x7fffffffu;
     const int e0 = p.m - p.L;
     const uint32_t thr = uint32_t(e0 + 127) << 23;
     const float scale = f32_from(uint32_t(p.L + 127) << 23);
+    const uint32_t sgn = (uint32_t)((int32_t)bits >> 31);
+    if (p.m <= kSignedMantissaF32) {
+#ifdef __CUDA_ARCH__
+        const float r = __fmaf_rn(x, scale, 12582912.0f);
+#else
+        const float r = std::fma(x, scale, 12582912.0f);
+#endif
+        const int sh = 23 - p.m;
+        const uint32_t c_log = (abits + ((1u << (sh - 1)) + (1u << 23) - thr)) >> sh;
+        return abits < thr ? (int32_t)(f32_bits(r) - 0x4b400000u) : (int32_t)((c_log ^ sgn) - sgn);
+    }
+    // m = 23: every mantissa bit is kept and the log region can pass the limit
 #ifdef __CUDA_ARCH__
     const float r = __fmaf_rn(f32_from(abits), scale, 8388608.0f);
 #else
     const float r = std::fma(f32_from(abits), scale, 8388608.0f);
 #endif
-    const uint32_t c_lin = f32_bits(r) - 0x4b000000u;
-    const int sh = 23 - p.m;
-    const uint32_t half = sh > 0 ? (1u << (sh - 1)) : 0u;
-    const uint32_t c_log = ((abits + half) >> sh) - (uint32_t(e0 + 127) << p.m) + (1u << p.m);
-    uint32_t c = abits < thr ? c_lin : c_log;
+    uint32_t c = abits < thr ? f32_bits(r) - 0x4b000000u : abits - thr + (1u << 23);
     if (abits >= thr && c > (uint32_t)kCodeLimit) c = (uint32_t)kCodeLimit;
-    const uint32_t sgn = (uint32_t)((int32_t)bits >> 31);
     return (int32_t)((c ^ sgn) - sgn);
 }
 
+// A code of the linear region (|q| <= 2^m, m <= kSignedMantissaF32): 1.5 * 2^23 + q
+// in units of 2^-L, minus 1.5 * 2^(23-L).
+__host__ __device__ inline float dequantize_linear(int32_t q, CodecParams p, float) {
+    const uint32_t eb = (uint32_t(150 - p.L) << 23) | 0x400000u;
+    return f32_from(eb + (uint32_t)q) - f32_from(eb);
+}
+
 __host__ __device__ inline float dequantize_fast_f32(int32_t q, CodecParams p) {
-    const uint32_t sgn = (uint32_t)(q >> 31);
-    const uint32_t c = ((uint32_t)q ^ sgn) - sgn;
+    const uint32_t c = (uint32_t)(q < 0 ? -q : q), sign = (uint32_t)q & 0x80000000u;
+    const int e0 = p.m - p.L;
+    if (p.m <= kSignedMantissaF32) {
+        const float lin = dequantize_linear(q, p, 0.0f);
+        const uint32_t lb = (c << (23 - p.m)) + (uint32_t(e0 + 126) << 23);
+        return c <= (1u << p.m) ? lin : f32_from(lb | sign);
+    }
     const uint32_t eb = uint32_t(150 - p.L) << 23;
     const float lin = f32_from(eb + c) - f32_from(eb);
-    const int e0 = p.m - p.L;
-    const uint32_t lb = (c + (uint32_t(e0 + 127) << p.m) - (1u << p.m)) << (23 - p.m);
-    const float a = c <= (1u << p.m) ? lin : f32_from(lb);
-    return f32_from(f32_bits(a) | (sgn & 0x80000000u));
+    const uint32_t lb = c + (uint32_t(e0 + 126) << 23);
+    return f32_from(f32_bits(c <= (1u << p.m) ? lin : f32_from(lb)) | sign);
+}
+
+// Whether every code of a chunk with this base and width lies in the linear
+// region, where the signed form above is the whole dequantisation.
+__host__ __device__ inline bool chunk_is_linear(int32_t base, uint32_t width, CodecParams p, double) {
+    return p.m <= kFastMantissaF64 && width <= 24 && base >= -(1 << p.m) &&
+           base + (int32_t)((1u << width) - 1u) <= (1 << p.m);
+}
+__host__ __device__ inline bool chunk_is_linear(int32_t base, uint32_t width, CodecParams p, float) {
+    return p.m <= kSignedMantissaF32 && width <= 24 && base >= -(1 << p.m) &&
+           base + (int32_t)((1u << width) - 1u) <= (1 << p.m);
 }
 
 // Dispatch on the precision and on the mantissa width (uniform per launch).

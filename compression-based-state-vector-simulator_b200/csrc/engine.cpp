@@ -1899,9 +1899,6 @@ qs_status qs_apply_circuit(qs_state *h) {
         a.final_pass = dp.final;
         a.exact_zero = (h->flags & QS_FLAG_EXACT_ZERO_TEST) ? 1 : 0;
         a.code_moves = dp.code_moves ? 1 : 0;
-        // complex64: passes of several sweeps measured faster with eight
-        // headers per batch, single-sweep (codec-bound) passes with four
-        a.header_batch = (!h->f64 && dp.nsweeps >= 2) ? 8 : 4;
         a.block_nz = h->block_nz;
         a.block_bytes = h->block_acc;
         a.error = h->error_dev;
@@ -2439,7 +2436,6 @@ qs_status qs_apply_dense_gate(qs_state *h, const uint32_t *targets, uint32_t k, 
     a.first_pass = 1;
     a.final_pass = 1;
     a.exact_zero = (h->flags & QS_FLAG_EXACT_ZERO_TEST) ? 1 : 0;
-    a.header_batch = 4;
     a.block_nz = h->block_nz;
     a.block_bytes = h->block_acc;
     a.error = h->error_dev;
@@ -2737,7 +2733,6 @@ qs_status qs_apply_diagonal_pauli_sum(qs_state *out, const qs_state *in, const u
         return fail(out, QS_ERR_CUDA, std::string("diagonal Pauli sum: ") + cudaGetErrorString(e));
     }
     qs::PassArgs a{};
-    a.header_batch = 4;
     a.n = (int)out->n;
     a.B = (int)out->B;
     a.C = C;

@@ -71,14 +71,30 @@ __device__ __forceinline__ uint64_t deposit_bits(uint32_t c, const int32_t *pos,
 }
 
 // ------------------------------------------------------------ tile layout
-// Element e of a tile lives at shared-memory slot swz(e) = e ^ ((e >> S1) & m):
-// an XOR of the low S1 bits with the next ones, so that a warp whose lanes
-// differ in any set of tile bits spreads over the banks.  m is limited to
-// bits below the chunk size, so an element never leaves its chunk's region.
+// Element e of a tile lives at shared-memory slot pos(e) = e + (e >> S1): one
+// slot of padding after every 128 bytes, so that a warp whose lanes differ in
+// bits above S1 spreads over the banks.  pos is additive over disjoint bits
+// (pos(a | b) = pos(a) + pos(b)), so a sweep's 16 offsets are sums of four
+// uniform numbers and a lane's components of a chunk lie at compile-time
+// distances from its first one.  (The XOR layout used before cost five
+// instructions a component in the codec and again in every sweep.)
 template <typename R> struct Layout;
 template <> struct Layout<double> { static constexpr int S1 = 3; };
 template <> struct Layout<float> { static constexpr int S1 = 4; };
 
+template <typename R>
+__host__ __device__ __forceinline__ constexpr int pos(int e) {
+    return e + (e >> Layout<R>::S1);
+}
+
+// Bytes of a tile of 2^nb amplitudes.
+template <typename R>
+__host__ __device__ __forceinline__ constexpr size_t tile_bytes(int nb) {
+    return ((size_t)pos<R>(1 << nb) * 2 * sizeof(R) + 15) / 16 * 16;
+}
+
+// The read-only kernels (expectation) keep an XOR layout: slot swz(e) = e ^
+// ((e >> S1) & m), m limited to bits below the chunk size.
 template <typename R>
 __host__ __device__ __forceinline__ int swizzle_mask(int C) {
     const int room = C - Layout<R>::S1;  // chunk bits above S1
@@ -267,46 +283,39 @@ __device__ __forceinline__ uint32_t outer_word(uint64_t base_amp, const int8_t *
 // function: it gets its own register allocation, apart from the codec phases
 // of the pass kernel, which measured faster; complex128 keeps them inlined.
 template <typename R, int RB>
-__device__ __forceinline__ void tile_sweeps_body(typename Cplx<R>::T *tile, int nb, int swm,
-                                                 const Sweep *__restrict__ sweeps, int nsweeps,
-                                                 const ROp *__restrict__ ops,
-                                                 const typename Cplx<R>::T *__restrict__ pool, uint32_t ow);
-template <typename R, int RB>
-__device__ __noinline__ void tile_sweeps_call(typename Cplx<R>::T *tile, int nb, int swm, const Sweep *__restrict__ sweeps,
-                            int nsweeps, const ROp *__restrict__ ops, const typename Cplx<R>::T *__restrict__ pool,
-                            uint32_t ow) { tile_sweeps_body<R, RB>(tile, nb, swm, sweeps, nsweeps, ops, pool, ow); }
-template <typename R, int RB>
-__device__ __forceinline__ void tile_sweeps(typename Cplx<R>::T *tile, int nb, int swm, const Sweep *__restrict__ sweeps,
-                            int nsweeps, const ROp *__restrict__ ops, const typename Cplx<R>::T *__restrict__ pool,
-                            uint32_t ow) {
-    if constexpr (sizeof(R) == 4) tile_sweeps_call<R, RB>(tile, nb, swm, sweeps, nsweeps, ops, pool, ow);
-    else tile_sweeps_body<R, RB>(tile, nb, swm, sweeps, nsweeps, ops, pool, ow);
-}
-template <typename R, int RB>
-__device__ __forceinline__ void tile_sweeps_body(typename Cplx<R>::T *tile, int nb, int swm, const Sweep *__restrict__ sweeps,
-                            int nsweeps, const ROp *__restrict__ ops, const typename Cplx<R>::T *__restrict__ pool,
-                            uint32_t ow) {
+__device__ __forceinline__ void tile_sweeps_body(typename Cplx<R>::T *tile, int nb, const Sweep *__restrict__ sweeps,
+                                                 int nsweeps, const ROp *__restrict__ ops,
+                                                 const typename Cplx<R>::T *__restrict__ pool, uint32_t ow) {
     using T = typename Cplx<R>::T;
     constexpr int NS = 1 << RB;
     const int groups = 1 << (nb - RB);
     const uint32_t wo = ow << nb;
     for (int w = 0; w < nsweeps; ++w) {
         const Sweep sw = sweeps[w];
-        int sb[RB], bm[RB];
+        int sb[RB], pb[RB];
 #pragma unroll
         for (int k = 0; k < RB; ++k) {
             sb[k] = sw.sbits[k];
-            bm[k] = 1 << sb[k];
+            pb[k] = pos<R>(1 << sb[k]);
         }
-        // offset of group element s: the OR of the masks of its set bits (s is
-        // a compile-time index, so each offset is a few ORs, no table)
-        auto off = [&](int s) {
-            int o = 0;
+        // offset of group element s: the sum of its set bits' offsets, in two
+        // halves so that an address is one three-input addition
+        constexpr int HB = RB / 2, HN = 1 << HB, TN = 1 << (RB - HB);
+        int olo[HN], ohi[TN];
 #pragma unroll
-            for (int k = 0; k < RB; ++k)
-                if ((s >> k) & 1) o |= bm[k];
-            return o;
-        };
+        for (int s = 0; s < HN; ++s) {
+            olo[s] = 0;
+#pragma unroll
+            for (int k = 0; k < HB; ++k)
+                if ((s >> k) & 1) olo[s] += pb[k];
+        }
+#pragma unroll
+        for (int s = 0; s < TN; ++s) {
+            ohi[s] = 0;
+#pragma unroll
+            for (int k = 0; k < RB - HB; ++k)
+                if ((s >> k) & 1) ohi[s] += pb[HB + k];
+        }
         for (int grp = threadIdx.x; grp < groups; grp += blockDim.x) {
             int base = grp;
 #pragma unroll
@@ -315,9 +324,10 @@ __device__ __forceinline__ void tile_sweeps_body(typename Cplx<R>::T *tile, int 
                 base = ((base >> t) << (t + 1)) | (base & ((1 << t) - 1));
             }
             const uint32_t W = (uint32_t)base | wo;
+            T *const g = tile + pos<R>(base);
             T v[NS];
 #pragma unroll
-            for (int s = 0; s < NS; ++s) v[s] = tile[swz<R>(base | off(s), swm)];
+            for (int s = 0; s < NS; ++s) v[s] = g[olo[s & (HN - 1)] + ohi[s >> HB]];
             T z = c_one<T>(), zh = c_one<T>();
             for (int k = sw.g0; k < sw.g1; ++k) {
                 const ROp o = ops[k];
@@ -328,10 +338,21 @@ __device__ __forceinline__ void tile_sweeps_body(typename Cplx<R>::T *tile, int 
                 for (int s = 0; s < NS; ++s) v[s] = cmul(z, v[s]);
             }
 #pragma unroll
-            for (int s = 0; s < NS; ++s) tile[swz<R>(base | off(s), swm)] = v[s];
+            for (int s = 0; s < NS; ++s) g[olo[s & (HN - 1)] + ohi[s >> HB]] = v[s];
         }
         __syncthreads();
     }
+}
+template <typename R, int RB>
+__device__ __noinline__ void tile_sweeps_call(typename Cplx<R>::T *tile, int nb, const Sweep *__restrict__ sweeps,
+                            int nsweeps, const ROp *__restrict__ ops, const typename Cplx<R>::T *__restrict__ pool,
+                            uint32_t ow) { tile_sweeps_body<R, RB>(tile, nb, sweeps, nsweeps, ops, pool, ow); }
+template <typename R, int RB>
+__device__ __forceinline__ void tile_sweeps(typename Cplx<R>::T *tile, int nb, const Sweep *__restrict__ sweeps,
+                            int nsweeps, const ROp *__restrict__ ops, const typename Cplx<R>::T *__restrict__ pool,
+                            uint32_t ow) {
+    if constexpr (sizeof(R) == 4) tile_sweeps_call<R, RB>(tile, nb, sweeps, nsweeps, ops, pool, ow);
+    else tile_sweeps_body<R, RB>(tile, nb, sweeps, nsweeps, ops, pool, ow);
 }
 
 // ------------------------------------------------------------ chunk codec
@@ -340,9 +361,14 @@ struct LinearSlot {
     __device__ __forceinline__ int operator()(int c) const { return c; }
 };
 
-// Component c of chunk `chunk` inside a swizzled tile.
+// Component c of the chunk that starts at tile element elem0.
 template <typename R>
 struct TileSlot {
+    int elem0;
+    __device__ __forceinline__ int operator()(int c) const { return 2 * pos<R>(elem0 + (c >> 1)) + (c & 1); }
+};
+template <typename R>
+struct XorSlot {
     int elem0, swm;
     __device__ __forceinline__ int operator()(int c) const { return 2 * swz<R>(elem0 + (c >> 1), swm) + (c & 1); }
 };
@@ -365,7 +391,7 @@ constexpr int kStageWords = (kMaxPerLane + 1) * 32;
 // copies, no registers, one commit group per call (empty for width 0).
 __device__ __forceinline__ void issue_payload(const uint32_t *__restrict__ arena, const ChunkMeta md, int per_lane,
                                               uint32_t *dst, int lane) {
-    const int rows = (int)(((uint32_t)per_lane * md.width + 31) >> 5);
+    const int rows = (int)(((uint32_t)per_lane * min(md.width, 32u) + 31) >> 5);
     const uint32_t sdst = (uint32_t)__cvta_generic_to_shared(dst);
     const char *gsrc = reinterpret_cast<const char *>(arena + (md.offset >> 2));
     for (int off = lane * 16; off < rows * 128; off += 32 * 16)
@@ -452,11 +478,8 @@ __device__ __forceinline__ void quantize_chunk(R *comp, int per_lane, CodecParam
         }
         __syncwarp();
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
     nz = __any_sync(0xffffffffu, nz);
     __syncwarp();
     *base_out = lo;
@@ -464,39 +487,255 @@ __device__ __forceinline__ void quantize_chunk(R *comp, int per_lane, CodecParam
     *nz_out = nz;
 }
 
+// Appends components of w bits to a lane's word stream, LSB first: the filled
+// bits sit at the top of acc (whatever is below them was written before), so
+// appending is one funnel shift and a word is complete after another.  The
+// branch is uniform in the warp (w is).
+struct WordPacker {
+    uint32_t acc = 0;
+    uint32_t filled = 0;      // bits of acc not written yet (< 32)
+    uint32_t *dst;
+    __device__ __forceinline__ explicit WordPacker(uint32_t *d) : dst(d) {}
+    __device__ __forceinline__ void add(uint32_t u, uint32_t w) {
+        if (filled + w >= 32) {
+            // the low 32 - filled bits of u complete the word
+            __stcs(dst, __funnelshift_rc(acc, u, 32 - filled));
+            dst += 32;
+            filled += w - 32;
+        } else {
+            filled += w;
+        }
+        acc = __funnelshift_rc(acc, u, w);
+    }
+    __device__ __forceinline__ void finish() {
+        if (filled) __stcs(dst, acc >> (32 - filled));
+    }
+};
+
 // Per-warp packing of int32 codes[lane + 32 i] to dst (layout in codec.cuh).
 __device__ __forceinline__ void pack_chunk(const int32_t *codes, int per_lane, int32_t base, uint32_t w,
                                            uint32_t *__restrict__ dst, int lane) {
     if (w == 0) return;
-    uint64_t buf = 0;
-    uint32_t nbits = 0, r = 0;
-    for (int i = 0; i < per_lane; ++i) {
-        const uint32_t u = (uint32_t)(codes[lane + 32 * i] - base);
-        buf |= (uint64_t)u << nbits;
-        nbits += w;
-        if (nbits >= 32) {
-            __stcs(dst + r * 32 + lane, (uint32_t)buf);
-            ++r;
-            buf >>= 32;
-            nbits -= 32;
+    WordPacker pk(dst + lane);
+    for (int i = 0; i < per_lane; ++i) pk.add((uint32_t)(codes[lane + 32 * i] - base), w);
+    pk.finish();
+}
+
+// The pass kernel's lane layout of a chunk: lane l handles amplitudes k + 16 i
+// with k = l & 15, i.e. payload streams 2k and 2k + 1, so that real and
+// imaginary part share their bit offsets, loads, stores and tile address;
+// lanes 0..15 take the first half of the i range, lanes 16..31 the second.
+// kPL: components per stream (2 .. 16 a power of two, 1 for 2^4-amplitude
+// chunks, whose second half has no lanes' work), 0 to use per_lane.
+template <int kPL>
+struct PairLanes {
+    static constexpr int H = kPL ? (kPL + 1) / 2 : kMaxPerLane / 2;   // amplitudes per lane, at most
+    int k, i0, n;                                                     // lane's stream pair, first i, amplitudes
+    __device__ __forceinline__ PairLanes(int per_lane, int lane) {
+        const int half = kPL ? H : (per_lane + 1) >> 1;
+        k = lane & 15;
+        i0 = (lane >> 4) * half;
+        n = (kPL > 1) ? H : min(half, per_lane - i0);
+    }
+};
+
+// The payload staging address inside a chunk's own tile region (cp.async
+// wants 16-byte alignment; the region has room for the largest payload).
+template <typename R>
+__device__ __forceinline__ uint32_t *chunk_stage(typename Cplx<R>::T *tile, int elem0) {
+    const size_t p = reinterpret_cast<size_t>(tile + pos<R>(elem0));
+    return reinterpret_cast<uint32_t *>((p + 15) & ~size_t(15));
+}
+
+// Per-warp decode of a chunk whose payload lies in the chunk's own tile region
+// (`src`, payload words; at most as many bytes as the values need): every lane
+// extracts its codes into registers, then the warp overwrites the region with
+// the values.  A chunk whose codes all lie in the linear region (its base and
+// width say so) skips the log region's half of the dequantisation.
+template <typename R, bool kCodes, int kPL>
+__device__ __forceinline__ void unpack_in_place(const ChunkMeta md, int per_lane, CodecParams p,
+                                                typename Cplx<R>::T *chunk_elem0, const uint32_t *src, int lane) {
+    using T = typename Cplx<R>::T;
+    const PairLanes<kPL> pl(per_lane, lane);
+    constexpr int H = PairLanes<kPL>::H;
+    T *const dst = chunk_elem0 + pos<R>(16 * pl.i0) + pos<R>(pl.k);
+    constexpr int kStep = 16 + (16 >> Layout<R>::S1);
+    // a width above 32 never comes from a pass or a checked import (unpack_chunk)
+    const uint32_t w = md.width > 32 ? 32u : md.width;
+    if (w == 0) {
+        T v;
+        v.x = v.y = kCodes ? code_as_value(md.base, R()) : dequantize_hot(md.base, p, R());
+#pragma unroll
+        for (int i = 0; i < H; ++i)
+            if (i < pl.n) dst[i * kStep] = v;
+        return;
+    }
+    const uint32_t mask = (w >= 32) ? 0xffffffffu : ((1u << w) - 1u);
+    const uint32_t *const s2 = src + 2 * pl.k;
+    int32_t q0[H], q1[H];
+    uint32_t bit = (uint32_t)pl.i0 * w;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        if (i < pl.n) {
+            const uint32_t *const row = s2 + (bit & ~31u);
+            const uint2 lo = *reinterpret_cast<const uint2 *>(row), hi = *reinterpret_cast<const uint2 *>(row + 32);
+            q0[i] = md.base + (int32_t)(__funnelshift_r(lo.x, hi.x, bit) & mask);
+            q1[i] = md.base + (int32_t)(__funnelshift_r(lo.y, hi.y, bit) & mask);
+            bit += w;
         }
     }
-    if (nbits > 0) __stcs(dst + r * 32 + lane, (uint32_t)buf);
+    __syncwarp();
+    if (!kCodes && chunk_is_linear(md.base, w, p, R())) {
+#pragma unroll
+        for (int i = 0; i < H; ++i)
+            if (i < pl.n) {
+                T v;
+                v.x = dequantize_linear(q0[i], p, R());
+                v.y = dequantize_linear(q1[i], p, R());
+                dst[i * kStep] = v;
+            }
+    } else {
+#pragma unroll
+        for (int i = 0; i < H; ++i)
+            if (i < pl.n) {
+                T v;
+                v.x = kCodes ? code_as_value(q0[i], R()) : dequantize_hot(q0[i], p, R());
+                v.y = kCodes ? code_as_value(q1[i], R()) : dequantize_hot(q1[i], p, R());
+                dst[i * kStep] = v;
+            }
+    }
 }
 
-__device__ __forceinline__ uint64_t apply_perm(const ChunkPerm &p, uint64_t c) {
+// A warp's output space: it takes `slab` bytes of the arena at a time (its
+// exact need when that is larger, or when slab is 0) and sub-allocates its
+// chunks, so encoding needs no other warp.  next, end: uniform in the warp.
+struct WarpArena {
+    unsigned long long next = 0, end = 0;
+    // Space for `bytes`; false (and the error flag set) when the arena is full.
+    __device__ __forceinline__ bool take(unsigned long long bytes, unsigned long long slab, unsigned long long *bump,
+                                         unsigned long long capacity, int32_t *error, int lane,
+                                         unsigned long long *off) {
+        if (next + bytes > end) {
+            const unsigned long long want = bytes > slab ? bytes : slab;
+            unsigned long long o = 0;
+            if (lane == 0) o = atomicAdd(bump, want);
+            o = __shfl_sync(0xffffffffu, o, 0);
+            if (o + want > capacity) {
+                if (lane == 0) atomicExch(error, 1);
+                return false;
+            }
+            next = o;
+            end = o + want;
+        }
+        *off = next;
+        next += bytes;
+        return true;
+    }
+};
+
+// Per-warp encoding of one tile chunk: quantise into registers, frame of
+// reference, space from the warp's arena slab, pack from registers.  Codes
+// never return to shared memory and no other warp is waited for.  A chunk
+// that finds the arena full gets a zero header (the error flag is set).
+// Returns the payload bytes; *nz: some amplitude is not zero (with exact_zero
+// the values are tested, else the codes: code 0 is exactly the value 0).
+template <typename R, bool kCodes, int kPL>
+__device__ __forceinline__ uint32_t encode_chunk(const typename Cplx<R>::T *chunk_elem0, int per_lane, int C,
+                                                 CodecParams p, bool exact_zero, int lane, WarpArena &wa,
+                                                 unsigned long long slab, unsigned long long *bump,
+                                                 unsigned long long capacity, int32_t *error,
+                                                 uint32_t *__restrict__ arena, ChunkMeta *__restrict__ out, bool *nz) {
+    using T = typename Cplx<R>::T;
+    const PairLanes<kPL> pl(per_lane, lane);
+    constexpr int H = PairLanes<kPL>::H;
+    const T *const src = chunk_elem0 + pos<R>(16 * pl.i0) + pos<R>(pl.k);
+    constexpr int kStep = 16 + (16 >> Layout<R>::S1);
+    int32_t q0[H], q1[H];
+    int32_t lo = INT_MAX, hi = INT_MIN;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        if (i < pl.n) {
+            const T v = src[i * kStep];
+            q0[i] = kCodes ? value_as_code(v.x) : quantize_hot(v.x, p);
+            q1[i] = kCodes ? value_as_code(v.y) : quantize_hot(v.y, p);
+            lo = __vimin3_s32(lo, q0[i], q1[i]);
+            hi = __vimax3_s32(hi, q0[i], q1[i]);
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (!kCodes && exact_zero) {
+        bool any = false;
+        for (int i = 0; i < pl.n; ++i) any |= src[i * kStep].x != R(0) || src[i * kStep].y != R(0);
+        *nz = __any_sync(0xffffffffu, any);
+    } else {
+        *nz = (lo | hi) != 0;
+    }
+    const uint32_t w = bit_length((uint32_t)hi - (uint32_t)lo);
+    const uint32_t bytes = (uint32_t)payload_bytes(C, w);
+    ChunkMeta md{0, 0, 0};
+    unsigned long long off = 0;
+    if (wa.take(bytes, slab, bump, capacity, error, lane, &off)) {
+        md.offset = off;
+        md.base = lo;
+        md.width = w;
+        if (w) {
+            // The word streams of a lane pair l, l + 16: the filled bits sit at
+            // the top of acc (what is below was written before), so appending a
+            // code is one funnel shift.  The upper lane starts with the bits
+            // that the lower lane's half leaves over.
+            uint32_t acc0 = 0, acc1 = 0;
+#pragma unroll
+            for (int i = 0; i < H; ++i)
+                if (i < pl.n) {
+                    q0[i] -= lo;
+                    q1[i] -= lo;
+                    acc0 = __funnelshift_rc(acc0, (uint32_t)q0[i], w);
+                    acc1 = __funnelshift_rc(acc1, (uint32_t)q1[i], w);
+                }
+            acc0 = __shfl_up_sync(0xffffffffu, acc0, 16);
+            acc1 = __shfl_up_sync(0xffffffffu, acc1, 16);
+            const uint32_t bit0 = (uint32_t)pl.i0 * w;
+            uint32_t filled = bit0 & 31u;
+            uint32_t *dst = arena + (off >> 2) + (bit0 & ~31u) + 2 * pl.k;
+#pragma unroll
+            for (int i = 0; i < H; ++i)
+                if (i < pl.n) {
+                    const uint32_t u0 = (uint32_t)q0[i], u1 = (uint32_t)q1[i];
+                    filled += w;
+                    if (filled >= 32) {
+                        // the low bits of the codes complete a word
+                        filled -= 32;
+                        __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(__funnelshift_rc(acc0, u0, w - filled),
+                                                                         __funnelshift_rc(acc1, u1, w - filled)));
+                        dst += 32;
+                    }
+                    acc0 = __funnelshift_rc(acc0, u0, w);
+                    acc1 = __funnelshift_rc(acc1, u1, w);
+                }
+            if (filled && pl.i0 + pl.n == per_lane && pl.n > 0)
+                __stcs(reinterpret_cast<uint2 *>(dst), make_uint2(acc0 >> (32 - filled), acc1 >> (32 - filled)));
+        }
+    }
+    if (lane == 0) *out = md;
+    return bytes;
+}
+
+// The bit moves of a chunk permutation (without its flips).
+__device__ __forceinline__ uint64_t move_perm(const ChunkPerm &p, uint64_t c) {
     uint64_t o = c & p.keep;
     for (int k = 0; k < p.nmove; ++k) o |= ((c >> p.src[k]) & 1ull) << p.dst[k];
-    return o ^ p.flip;
+    return o;
 }
 
-size_t pass_smem_bytes(bool f64, int nb, int j) {
-    const size_t tile = (f64 ? 16 : 8) << nb;
-    const size_t stage = (size_t)(kSweepThreads / 32) * kStageWords * 4;
-    const size_t tables = ((size_t)3 * 4 << j) + 8;
-    const size_t offs = (size_t)8 << j;
-    const size_t headers = sizeof(ChunkMeta) << j;
-    return tile + stage + ((tables + 7) / 8) * 8 + offs + headers;
+__device__ __forceinline__ uint64_t apply_perm(const ChunkPerm &p, uint64_t c) { return move_perm(p, c) ^ p.flip; }
+
+// Shared memory of one pass_kernel CTA: the tile, one payload row that the
+// last chunk's unpack may read ahead, the chunk headers, and the tile's term
+// coefficients when the pass applies a diagonal sum.
+size_t pass_smem_bytes(bool f64, int nb, int j, int diag_terms) {
+    return (f64 ? tile_bytes<double>(nb) : tile_bytes<float>(nb)) + 128 + (sizeof(ChunkMeta) << j) +
+           ((size_t)16 << j) + (size_t)16 * diag_terms;
 }
 
 // ------------------------------------------------------------ diagonal Pauli sum
@@ -504,8 +743,7 @@ size_t pass_smem_bytes(bool f64, int nb, int j) {
 // of each term is folded into its coefficient once per tile (s_dc, 2 doubles
 // per term, written and read by the whole CTA between barriers).
 template <typename R>
-__device__ void tile_diag_sum(typename Cplx<R>::T *tile, int nb, int swm, const DiagSum &d, uint64_t base_amp,
-                              double *s_dc) {
+__device__ void tile_diag_sum(typename Cplx<R>::T *tile, int nb, const DiagSum &d, uint64_t base_amp, double *s_dc) {
     using T = typename Cplx<R>::T;
     for (int t = threadIdx.x; t < d.nterms; t += blockDim.x) {
         const double sg = (__popcll(base_amp & d.terms[t].zo) & 1) ? -1.0 : 1.0;
@@ -520,7 +758,7 @@ __device__ void tile_diag_sum(typename Cplx<R>::T *tile, int nb, int swm, const 
             hr = fma(sg, s_dc[2 * t], hr);
             hi = fma(sg, s_dc[2 * t + 1], hi);
         }
-        T &v = tile[swz<R>(e, swm)];
+        T &v = tile[pos<R>(e)];
         const double vr = (double)v.x, vi = (double)v.y;
         v.x = (R)(hr * vr - hi * vi);
         v.y = (R)(hr * vi + hi * vr);
@@ -528,244 +766,111 @@ __device__ void tile_diag_sum(typename Cplx<R>::T *tile, int nb, int swm, const 
     __syncthreads();
 }
 
-static_assert((kSweepThreads / 32) * kStageWords * 4 >= 2 * kMaxDiagTerms * sizeof(double),
-              "the pass kernel's decode staging holds the diagonal-sum coefficients");
-
-// ------------------------------------------------------------ pass kernel
-// Whether a warp loads all its chunk headers at once and copies its next
-// chunk's payload while it unpacks the current one (complex128, measured
-// faster there), or loads headers four at a time and copies each payload
-// just before unpacking it (complex64, measured faster there).
-template <typename R>
-constexpr bool kPrefetchDecode = sizeof(R) == 8;
-
 // ------------------------------------------------------------ pass kernel
 // kCodes: every op of the pass only moves amplitudes (X / SWAP register
 // moves, chunk permutations), so the tile holds the quantised codes
 // themselves and the pass skips dequantisation and quantisation.
-// kHB: complex64 chunk headers loaded per warp batch (4 or 8).
 // kC, kJ: the chunk log2 and the tile qubits above the chunk when known at
 // compile time, 0 to read them from the args.
-template <typename R, int RB, bool kCodes, int kHB, int kC, int kJ>
+//
+// A warp decodes and encodes the same chunks of every tile, so the CTA meets
+// only around the sweeps: between a tile's encode and the next one's decode
+// its warps run apart.  All payloads of a warp's chunks are copied at once,
+// each into its chunk's own tile region (no staging buffer).
+template <typename R, int RB, bool kCodes, int kC, int kJ>
 __global__ void __launch_bounds__(kSweepThreads, 3) pass_kernel(const PassArgs a) {
     using T = typename Cplx<R>::T;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ unsigned long long s_tile_off, s_next, s_slab_end;
-    __shared__ int s_flag;
     __shared__ int32_t s_tq[kMaxTileQubits];
     __shared__ int8_t s_oq[kMaxOuterSel];
+    __shared__ int s_err;
+    if (threadIdx.x == 0) s_err = *reinterpret_cast<volatile int32_t *>(a.error);
     if (threadIdx.x < kMaxTileQubits) s_tq[threadIdx.x] = a.tq[threadIdx.x];
     if (threadIdx.x < kMaxOuterSel) s_oq[threadIdx.x] = a.outer_q[threadIdx.x];
-    if (threadIdx.x == 0) {
-        s_next = 0;
-        s_slab_end = 0;
-    }
     __syncthreads();
+    if (s_err) return;  // an earlier pass overflowed its arena: its store is not valid
 
     const int C = kC ? kC : a.C, j = kJ ? kJ : a.j, nb = C + j;
+    constexpr int kPL = kC ? (2 << kC) / 32 : 0;
     const int nchunks = 1 << j;
     const int ncomp = 2 << C;
     const int per_lane = ncomp >> 5;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int blk_shift = a.B - C;
-    const int swm = swizzle_mask<R>(C);
 
     T *tile = reinterpret_cast<T *>(smem);
-    uint32_t *stage_all = reinterpret_cast<uint32_t *>(smem + (sizeof(T) << nb));
-    uint32_t *wstage = stage_all + warp * kStageWords;
-    int32_t *s_base = reinterpret_cast<int32_t *>(stage_all + nwarps * kStageWords);
-    uint32_t *s_width = reinterpret_cast<uint32_t *>(s_base + nchunks);
-    uint32_t *s_nz = s_width + nchunks;
-    unsigned long long *s_off = reinterpret_cast<unsigned long long *>(
-        reinterpret_cast<unsigned char *>(s_base) + ((((size_t)3 * 4 << j) + 8 + 7) / 8) * 8);
-    ChunkMeta *s_md = reinterpret_cast<ChunkMeta *>(s_off + nchunks);
+    ChunkMeta *s_md = reinterpret_cast<ChunkMeta *>(smem + tile_bytes<R>(nb) + 128);
+    // chunk c of a tile: its index bits, and where the pass stores it (the
+    // chunk permutation acts on each index bit on its own, so both are ORed
+    // with the tile's part)
+    uint64_t *s_in = reinterpret_cast<uint64_t *>(s_md + nchunks), *s_out = s_in + nchunks;
+    for (int c = threadIdx.x; c < nchunks; c += blockDim.x) {
+        s_in[c] = deposit_bits((uint32_t)c, s_tq, j);
+        s_out[c] = move_perm(a.perm, s_in[c]);
+    }
+    __syncthreads();
+    const unsigned long long slab = a.slab / (kSweepThreads / 32) / 128 * 128;  // per warp
 
+    WarpArena wa;
     unsigned long long rd = 0, wr = 0, ntiles = 0;
 
     for (uint64_t tile_id = blockIdx.x; tile_id < a.n_tiles; tile_id += gridDim.x) {
         const uint64_t chunk_base = insert_zero_bits(tile_id, s_tq, j);
         const uint64_t block0 = chunk_base >> blk_shift;
         if (!a.group_active[a.block_to_group[block0]]) continue;  // uniform in the CTA
-        if (threadIdx.x == 0) s_flag = *reinterpret_cast<volatile int32_t *>(a.error);
-        __syncthreads();
-        if (s_flag) break;
         ++ntiles;
 
-        if constexpr (!kPrefetchDecode<R>) {
-            // ---- decode: the headers of kHB of the warp's chunks are
-            // loaded together, then the chunks are unpacked one by one
-            constexpr int HB = kHB;
-            for (int c0 = warp; c0 < nchunks; c0 += HB * nwarps) {
-                ChunkMeta md[HB];
-                bool zero[HB];
-#pragma unroll
-                for (int b = 0; b < HB; ++b) {
-                    const int c = c0 + b * nwarps;
-                    md[b] = ChunkMeta{0, 0, 0};
-                    zero[b] = true;
-                    if (c < nchunks) {
-                        const uint64_t chunk = chunk_base | deposit_bits((uint32_t)c, s_tq, j);
-                        if (!a.first_pass || a.mask[chunk >> blk_shift]) {
-                            md[b] = a.meta_in[chunk];
-                            zero[b] = false;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int b = 0; b < HB; ++b) {
-                    const int c = c0 + b * nwarps;
-                    if (c >= nchunks) break;
-                    R *comp = reinterpret_cast<R *>(tile) + (size_t)c * ncomp;
-                    if (zero[b]) {
-                        for (int i = 0; i < per_lane; ++i) comp[lane + 32 * i] = R(0);
-                        continue;
-                    }
-                    decode_chunk<R, TileSlot<R>, kCodes>(a.arena_in, md[b], per_lane, a.codec,
-                                                         reinterpret_cast<R *>(tile), wstage, lane,
-                                                         TileSlot<R>{c << C, swm});
-                    if (lane == 0) rd += payload_bytes(C, md[b].width) + sizeof(ChunkMeta);
-                }
+        // ---- decode.  A warp's lanes load the headers of its chunks at once
+        // (a chunk of a zero block reads as width 0, base 0: zeros), the warp
+        // starts every payload copy, then unpacks chunk by chunk.
+        for (int c = warp + lane * nwarps; c < nchunks; c += 32 * nwarps) {
+            ChunkMeta md{0, 0, 0};
+            const uint64_t chunk = chunk_base | s_in[c];
+            if (!a.first_pass || a.mask[chunk >> blk_shift]) {
+                md = a.meta_in[chunk];
+                rd += payload_bytes(C, md.width) + sizeof(ChunkMeta);
             }
-        } else {
-            // ---- decode.  A warp's lanes load the headers of all of the
-            // warp's chunks at once (a chunk of a zero block reads as width 0,
-            // base 0: zeros).  The warp then walks its chunks and copies the
-            // next chunk's payload with cp.async while it unpacks the current
-            // one; the two payload buffers are the warp's staging area and
-            // the tile region of the warp's last chunk, which nothing uses
-            // until that chunk is unpacked.
-            for (int c = warp + lane * nwarps; c < nchunks; c += 32 * nwarps) {
-                ChunkMeta md{0, 0, 0};
-                const uint64_t chunk = chunk_base | deposit_bits((uint32_t)c, s_tq, j);
-                if (!a.first_pass || a.mask[chunk >> blk_shift]) {
-                    md = a.meta_in[chunk];
-                    rd += payload_bytes(C, md.width) + sizeof(ChunkMeta);
-                }
-                s_md[c] = md;
-            }
-            __syncwarp();
-            const int m = warp < nchunks ? (nchunks - warp + nwarps - 1) / nwarps : 0;
-            if (m > 0) {
-                uint32_t *bufR = reinterpret_cast<uint32_t *>(reinterpret_cast<R *>(tile) +
-                                                              (size_t)(warp + (m - 1) * nwarps) * ncomp);
-                issue_payload(a.arena_in, s_md[warp], per_lane, wstage, lane);
-                for (int i = 0; i < m; ++i) {
-                    const int c = warp + i * nwarps;
-                    uint32_t *cur = (i < m - 1 && (i & 1)) ? bufR : wstage;
-                    uint32_t *nxt = (i + 1 < m - 1 && ((i + 1) & 1)) ? bufR : wstage;
-                    const bool pre = i + 1 < m && nxt != cur;
-                    if (pre) {
-                        issue_payload(a.arena_in, s_md[c + nwarps], per_lane, nxt, lane);
-                        cp_async_wait<1>();
-                    } else {
-                        cp_async_wait<0>();
-                    }
-                    __syncwarp();
-                    unpack_chunk<R, TileSlot<R>, kCodes>(s_md[c], per_lane, a.codec, reinterpret_cast<R *>(tile), cur,
-                                                         lane, TileSlot<R>{c << C, swm});
-                    __syncwarp();
-                    if (i + 1 < m && !pre) issue_payload(a.arena_in, s_md[c + nwarps], per_lane, nxt, lane);
-                }
-            }
+            s_md[c] = md;
+        }
+        __syncwarp();
+        for (int c = warp; c < nchunks; c += nwarps)
+            issue_payload(a.arena_in, s_md[c], per_lane, chunk_stage<R>(tile, c << C), lane);
+        cp_async_wait<0>();
+        __syncwarp();
+        for (int c = warp; c < nchunks; c += nwarps) {
+            unpack_in_place<R, kCodes, kPL>(s_md[c], per_lane, a.codec, tile + pos<R>(c << C),
+                                            chunk_stage<R>(tile, c << C), lane);
         }
         __syncthreads();
 
         // ---- gates
-        tile_sweeps<R, RB>(tile, nb, swm, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool),
+        tile_sweeps<R, RB>(tile, nb, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool),
                            outer_word(chunk_base << C, s_oq, a.nouter));
-        // the decode staging area is free here: it holds the tile's term coefficients
         if constexpr (!kCodes) {
             if (a.diag.nterms)
-                tile_diag_sum<R>(tile, nb, swm, a.diag, chunk_base << C, reinterpret_cast<double *>(stage_all));
+                tile_diag_sum<R>(tile, nb, a.diag, chunk_base << C, reinterpret_cast<double *>(s_out + nchunks));
         }
 
-        // ---- quantise (codes replace values in shared memory)
+        // ---- quantise, reserve and pack, chunk by chunk
+        const uint64_t out_base = move_perm(a.perm, chunk_base);
         for (int c = warp; c < nchunks; c += nwarps) {
-            R *comp = reinterpret_cast<R *>(tile) + (size_t)c * ncomp;
-            int32_t base;
-            uint32_t width;
+            const uint64_t chunk = (out_base | s_out[c]) ^ a.perm.flip;
             bool nz;
-            quantize_chunk<R, TileSlot<R>, kCodes>(reinterpret_cast<R *>(tile), per_lane, a.codec, a.exact_zero != 0,
-                                                   lane, &base, &width, &nz, TileSlot<R>{c << C, swm},
-                                                   reinterpret_cast<int32_t *>(comp));
-            if (lane == 0) {
-                s_base[c] = base;
-                s_width[c] = width;
-                s_nz[c] = nz ? 1u : 0u;
+            const uint32_t bytes = encode_chunk<R, kCodes, kPL>(tile + pos<R>(c << C), per_lane, C, a.codec,
+                                                                a.exact_zero != 0, lane, wa, slab, a.bump, a.capacity,
+                                                                a.error, a.arena_out, a.meta_out + chunk, &nz);
+            wr += bytes + sizeof(ChunkMeta);
+            if (a.final_pass && lane == 0) {
+                const uint64_t blk = chunk >> blk_shift;
+                if (nz) atomicOr(&a.block_nz[blk], 1u);
+                atomicAdd(&a.block_bytes[blk], (unsigned long long)(bytes + sizeof(ChunkMeta)));
             }
         }
-        __syncthreads();
-
-        // ---- reserve the tile's output bytes with one atomic: warp 0 scans
-        // the chunk sizes (each lane a run of consecutive chunks)
-        if (warp == 0) {
-            const int per = (nchunks + 31) >> 5;
-            const int c0 = lane * per;
-            unsigned long long mine = 0;
-            for (int c = c0; c < c0 + per && c < nchunks; ++c) mine += payload_bytes(C, s_width[c]);
-            unsigned long long incl = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            unsigned long long run = incl - mine;
-            for (int c = c0; c < c0 + per && c < nchunks; ++c) {
-                s_off[c] = run;
-                run += payload_bytes(C, s_width[c]);
-            }
-            const unsigned long long total = __shfl_sync(0xffffffffu, incl, 31);
-            if (lane == 0) {
-                // the tile goes at the CTA's next free byte of its current
-                // slab; one that does not fit takes a new slab of a.slab
-                // bytes (or exactly its own size) from the arena, so most
-                // tiles reserve without touching the shared counter
-                unsigned long long off = s_next;
-                s_flag = 0;
-                if (a.slab == 0 || off + total > s_slab_end) {
-                    const unsigned long long want = total > a.slab ? total : a.slab;
-                    off = atomicAdd(a.bump, want);
-                    if (off + want > a.capacity) {
-                        atomicExch(a.error, 1);
-                        s_flag = 1;
-                    }
-                    s_slab_end = off + want;
-                }
-                s_tile_off = off;
-                s_next = off + total;
-                wr += total + (unsigned long long)nchunks * sizeof(ChunkMeta);
-            }
-        }
-        __syncthreads();
-        if (s_flag) break;
-
-        // ---- pack and store
-        for (int c = warp; c < nchunks; c += nwarps) {
-            const uint64_t chunk = apply_perm(a.perm, chunk_base | deposit_bits((uint32_t)c, s_tq, j));
-            const int32_t *codes = reinterpret_cast<const int32_t *>(reinterpret_cast<R *>(tile) + (size_t)c * ncomp);
-            const unsigned long long off = s_tile_off + s_off[c];
-            const uint32_t w = s_width[c];
-            pack_chunk(codes, per_lane, s_base[c], w, a.arena_out + (off >> 2), lane);
-            if (lane == 0) {
-                ChunkMeta md;
-                md.offset = off;
-                md.base = s_base[c];
-                md.width = w;
-                a.meta_out[chunk] = md;
-                if (a.final_pass) {
-                    const uint64_t blk = chunk >> blk_shift;
-                    if (s_nz[c]) atomicOr(&a.block_nz[blk], 1u);
-                    atomicAdd(&a.block_bytes[blk], (unsigned long long)(payload_bytes(C, w) + sizeof(ChunkMeta)));
-                }
-            }
-        }
-        __syncthreads();
+        __syncwarp();
     }
     if (rd) atomicAdd(&a.stats[0], rd);
-    if (threadIdx.x == 0) {
-        if (wr) atomicAdd(&a.stats[1], wr);
-        if (ntiles) atomicAdd(&a.stats[2], ntiles);
-    }
+    if (lane == 0 && wr) atomicAdd(&a.stats[1], wr);
+    if (threadIdx.x == 0 && ntiles) atomicAdd(&a.stats[2], ntiles);
 }
 
 // ------------------------------------------------------------ staged pass kernel
@@ -881,7 +986,7 @@ __host__ __device__ inline StagedLayout staged_layout(bool f64, int C, int j, ui
     StagedLayout L{};
     const size_t nch = (size_t)1 << j;
     size_t o = 0;
-    L.tile = o;  o += align128((f64 ? 16 : 8) << (C + j));
+    L.tile = o;  o += align128(f64 ? tile_bytes<double>(C + j) : tile_bytes<float>(C + j));
     const size_t stage = align128(staged_stage_bytes(C, j));
     L.buf0 = o;  o += stage;
     L.buf1 = o;  o += stage;
@@ -997,7 +1102,7 @@ __device__ __forceinline__ uint32_t dense_row_base(uint32_t o, uint32_t gmask, i
 // (hi, lo), dep: pattern offsets, d_tmem: the accumulator, bar: the MMA
 // mbarrier with its phase parity.  Returns false when the MMAs did not
 // complete within the bounded wait.
-__device__ bool tile_dense_k_tc(float2 *tile, int nb, int swm, int k, const int32_t *dep, uint32_t gmask,
+__device__ bool tile_dense_k_tc(float2 *tile, int nb, int k, const int32_t *dep, uint32_t gmask,
                                 float *aop, const float *bop, uint32_t d_tmem, uint64_t *bar, uint32_t parity) {
     const int K = 1 << k;              // complex patterns
     const int Kp = 2 * K;              // realified columns
@@ -1015,7 +1120,7 @@ __device__ bool tile_dense_k_tc(float2 *tile, int nb, int swm, int k, const int3
             float re[4], im[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float2 v = tile[swz<float>((int)(base | (uint32_t)dep[r4 + i]), swm)];
+                const float2 v = tile[pos<float>((int)(base | (uint32_t)dep[r4 + i]))];
                 re[i] = v.x;
                 im[i] = v.y;
             }
@@ -1073,7 +1178,7 @@ __device__ bool tile_dense_k_tc(float2 *tile, int nb, int swm, int k, const int3
             tmem_wait_ld();
 #pragma unroll
             for (int i = 0; i < 16; ++i)
-                if (c0 + i < K) tile[swz<float>((int)(base | (uint32_t)dep[c0 + i]), swm)] = make_float2(re[i], im[i]);
+                if (c0 + i < K) tile[pos<float>((int)(base | (uint32_t)dep[c0 + i]))] = make_float2(re[i], im[i]);
         }
     }
     tmem_fence_before();
@@ -1082,7 +1187,7 @@ __device__ bool tile_dense_k_tc(float2 *tile, int nb, int swm, int k, const int3
 }
 
 // complex128: y = G x per tile column on the CUDA cores (G in shared memory).
-__device__ void tile_dense_k_f64(double2 *tile, int nb, int swm, int k, const int32_t *dep, uint32_t gmask,
+__device__ void tile_dense_k_f64(double2 *tile, int nb, int k, const int32_t *dep, uint32_t gmask,
                                  const double2 *g) {
     const int K = 1 << k;
     const int rows = 1 << (nb - k);
@@ -1091,13 +1196,13 @@ __device__ void tile_dense_k_f64(double2 *tile, int nb, int swm, int k, const in
         double2 x[1 << kMaxDenseK];
 #pragma unroll
         for (int c = 0; c < (1 << kMaxDenseK); ++c)
-            if (c < K) x[c] = tile[swz<double>((int)(base | (uint32_t)dep[c]), swm)];
+            if (c < K) x[c] = tile[pos<double>((int)(base | (uint32_t)dep[c]))];
         for (int r = 0; r < K; ++r) {
             double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
             for (int c = 0; c < (1 << kMaxDenseK); ++c)
                 if (c < K) acc = cfma(g[r * K + c], x[c], acc);
-            tile[swz<double>((int)(base | (uint32_t)dep[r]), swm)] = acc;
+            tile[pos<double>((int)(base | (uint32_t)dep[r]))] = acc;
         }
     }
     __syncthreads();
@@ -1125,7 +1230,6 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
     const int per_lane = ncomp >> 5;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int blk_shift = a.B - C;
-    const int swm = swizzle_mask<R>(C);
     const uint32_t nblk = 1u << (a.n - a.B);
     const bool smask = nblk <= kMaxSmemBlocks;
     const uint32_t mask_words = smask ? (nblk + 31) / 32 : 0;
@@ -1304,7 +1408,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
         for (int c = warp; c < nchunks; c += nwarps) {
             const ChunkMeta md = hdr(slot)[c];
             unpack_chunk<R, TileSlot<R>, kCodes>(md, per_lane, a.codec, reinterpret_cast<R *>(tile),
-                                                 buf(slot) + (poff(slot)[c] >> 2), lane, TileSlot<R>{c << C, swm});
+                                                 buf(slot) + (poff(slot)[c] >> 2), lane, TileSlot<R>{c << C});
             if (lane == 0) {
                 const uint64_t chunk = chunk_base | deposit_bits((uint32_t)c, s_tq, j);
                 if (!a.first_pass || block_stored(chunk >> blk_shift))
@@ -1318,7 +1422,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
         // ---- gates
         if constexpr (kDense) {
             if constexpr (sizeof(R) == 4) {
-                const bool done = tile_dense_k_tc(reinterpret_cast<float2 *>(tile), nb, swm, a.dense.k, dense_dep,
+                const bool done = tile_dense_k_tc(reinterpret_cast<float2 *>(tile), nb, a.dense.k, dense_dep,
                                                   dense_gmask, reinterpret_cast<float *>(smem + Ly.dense_a),
                                                   reinterpret_cast<const float *>(smem + Ly.dense_b), s_tmem,
                                                   &s_mma, mma_phase);
@@ -1329,27 +1433,27 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
                 }
                 mma_phase ^= 1u;
             } else {
-                tile_dense_k_f64(reinterpret_cast<double2 *>(tile), nb, swm, a.dense.k, dense_dep, dense_gmask,
+                tile_dense_k_f64(reinterpret_cast<double2 *>(tile), nb, a.dense.k, dense_dep, dense_gmask,
                                  reinterpret_cast<const double2 *>(smem + Ly.dense_b));
             }
         } else {
-            tile_sweeps<R, kRegBits>(tile, nb, swm, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool),
+            tile_sweeps<R, kRegBits>(tile, nb, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool),
                                      outer_word(chunk_base << C, s_oq, a.nouter));
             if constexpr (!kCodes) {
                 // buf(slot) is free here: it holds the tile's term coefficients
                 if (a.diag.nterms)
-                    tile_diag_sum<R>(tile, nb, swm, a.diag, chunk_base << C, reinterpret_cast<double *>(buf(slot)));
+                    tile_diag_sum<R>(tile, nb, a.diag, chunk_base << C, reinterpret_cast<double *>(buf(slot)));
             }
         }
 
         // ---- quantise (codes replace values in shared memory)
         for (int c = warp; c < nchunks; c += nwarps) {
-            R *comp = reinterpret_cast<R *>(tile) + (size_t)c * ncomp;
+            R *comp = reinterpret_cast<R *>(tile + pos<R>(c << C));
             int32_t base;
             uint32_t width;
             bool nz;
             quantize_chunk<R, TileSlot<R>, kCodes>(reinterpret_cast<R *>(tile), per_lane, a.codec, a.exact_zero != 0,
-                                                   lane, &base, &width, &nz, TileSlot<R>{c << C, swm},
+                                                   lane, &base, &width, &nz, TileSlot<R>{c << C},
                                                    reinterpret_cast<int32_t *>(comp));
             if (lane == 0) {
                 s_base[c] = base;
@@ -1400,7 +1504,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
         // ---- pack and store
         for (int c = warp; c < nchunks; c += nwarps) {
             const uint64_t chunk = apply_perm(a.perm, chunk_base | deposit_bits((uint32_t)c, s_tq, j));
-            const int32_t *codes = reinterpret_cast<const int32_t *>(reinterpret_cast<R *>(tile) + (size_t)c * ncomp);
+            const int32_t *codes = reinterpret_cast<const int32_t *>(tile + pos<R>(c << C));
             const unsigned long long off = s_tile_off + s_off[c];
             const uint32_t w = s_width[c];
             pack_chunk(codes, per_lane, s_base[c], w, a.arena_out + (off >> 2), lane);
@@ -1498,7 +1602,6 @@ __global__ void __launch_bounds__(kSweepThreads, 3) dense_pass_kernel(const Dens
     const int C = kC ? kC : a.C, j = kJ ? kJ : a.j, nb = C + j;
     const int size = 1 << nb;
     const int cmask = (1 << C) - 1;
-    const int swm = swizzle_mask<R>(C);
     __shared__ int32_t s_tq[kMaxTileQubits];
     __shared__ int8_t s_oq[kMaxOuterSel];
     if (threadIdx.x < kMaxTileQubits) s_tq[threadIdx.x] = a.tq[threadIdx.x];
@@ -1508,14 +1611,14 @@ __global__ void __launch_bounds__(kSweepThreads, 3) dense_pass_kernel(const Dens
         const uint64_t chunk_base = insert_zero_bits(tile_id, s_tq, j);
         for (int e = threadIdx.x; e < size; e += blockDim.x) {
             const uint64_t amp = ((chunk_base | deposit_bits((uint32_t)(e >> C), s_tq, j)) << C) | (uint64_t)(e & cmask);
-            tile[swz<R>(e, swm)] = st[amp];
+            tile[pos<R>(e)] = st[amp];
         }
         __syncthreads();
-        tile_sweeps<R, RB>(tile, nb, swm, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool),
+        tile_sweeps<R, RB>(tile, nb, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool),
                            outer_word(chunk_base << C, s_oq, a.nouter));
         for (int e = threadIdx.x; e < size; e += blockDim.x) {
             const uint64_t amp = ((chunk_base | deposit_bits((uint32_t)(e >> C), s_tq, j)) << C) | (uint64_t)(e & cmask);
-            st[amp] = tile[swz<R>(e, swm)];
+            st[amp] = tile[pos<R>(e)];
         }
         __syncthreads();
     }
@@ -1952,7 +2055,7 @@ __global__ void __launch_bounds__(kExpectThreads) expect_kernel(const ExpectArgs
                     continue;
                 }
                 decode_chunk<R>(arena, meta[chunk], per_lane, a.codec, reinterpret_cast<R *>(dst), wstage, lane,
-                                TileSlot<R>{c << C, swm});
+                                XorSlot<R>{c << C, swm});
             }
         }
         __syncthreads();
@@ -2686,25 +2789,26 @@ int sm_count() {
     return g_sm_count;
 }
 
-template <typename R, int RB, bool kCodes, int kHB, int kC, int kJ>
+template <typename R, int RB, bool kCodes, int kC, int kJ>
 static cudaError_t launch_pass_kc(const PassArgs &a, cudaStream_t s) {
     const int nb = a.C + a.j;
-    const size_t smem = pass_smem_bytes(sizeof(R) == 8, nb, a.j);
-    cudaError_t e = ensure_dyn_smem(pass_kernel<R, RB, kCodes, kHB, kC, kJ>, smem);
+    const size_t smem = pass_smem_bytes(sizeof(R) == 8, nb, a.j, a.diag.nterms);
+    cudaError_t e = ensure_dyn_smem(pass_kernel<R, RB, kCodes, kC, kJ>, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<R, RB, kCodes, kHB, kC, kJ>, kSweepThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<R, RB, kCodes, kC, kJ>, kSweepThreads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     uint64_t grid = (uint64_t)per_sm * sm_count();
     if (grid > a.n_tiles) grid = a.n_tiles;
     if (grid == 0) grid = 1;
-    // arena slabs per CTA when the arena can spare 8 of them per CTA
+    // arena slabs per CTA (shared out to its warps) when the arena can spare
+    // 8 of them per CTA
     PassArgs b = a;
     const char *env = std::getenv("QOMPSIM_SLAB_BYTES");
     const uint64_t slab = env ? (uint64_t)std::strtoull(env, nullptr, 10) : (uint64_t)kArenaSlabBytes;
     b.slab = (slab && a.capacity / grid >= 8 * slab) ? (slab + 127) / 128 * 128 : 0;
-    pass_kernel<R, RB, kCodes, kHB, kC, kJ><<<(unsigned)grid, kSweepThreads, smem, s>>>(b);
+    pass_kernel<R, RB, kCodes, kC, kJ><<<(unsigned)grid, kSweepThreads, smem, s>>>(b);
     return cudaGetLastError();
 }
 
@@ -2713,12 +2817,12 @@ static cudaError_t launch_pass_kc(const PassArgs &a, cudaStream_t s) {
 // above the chunk) are compile-time constants of their instantiation: the
 // per-lane counts, chunk and group counts, offsets and swizzle mask then fold
 // into the code (measured 12-19 % faster than reading them from the args).
-template <typename R, int RB, bool kCodes, int kHB>
+template <typename R, int RB, bool kCodes>
 static cudaError_t launch_pass_t(const PassArgs &a, cudaStream_t s) {
     constexpr int J = sizeof(R) == 8 ? 4 : 5;
-    if (a.C == kMaxChunkLog2 && a.j == J) return launch_pass_kc<R, RB, kCodes, kHB, kMaxChunkLog2, J>(a, s);
-    return a.C == kMaxChunkLog2 ? launch_pass_kc<R, RB, kCodes, kHB, kMaxChunkLog2, 0>(a, s)
-                                : launch_pass_kc<R, RB, kCodes, kHB, 0, 0>(a, s);
+    if (a.C == kMaxChunkLog2 && a.j == J) return launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, J>(a, s);
+    return a.C == kMaxChunkLog2 ? launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, 0>(a, s)
+                                : launch_pass_kc<R, RB, kCodes, 0, 0>(a, s);
 }
 
 template <typename R, bool kCodes, bool kDense, int kC, int kJ>
@@ -2758,7 +2862,6 @@ static cudaError_t launch_staged_t(const PassArgs &a, cudaStream_t s) {
 cudaError_t launch_pass(bool f64, const PassArgs &a, int, cudaStream_t s) {
     if (a.rb != kRegBits || a.C + a.j < kRegBits || a.diag.nterms > kMaxDiagTerms) return cudaErrorInvalidValue;
     if (a.code_moves && a.diag.nterms) return cudaErrorInvalidValue;
-    if (a.header_batch != 4 && a.header_batch != 8) return cudaErrorInvalidValue;
     if (a.dense.k) {
         // one dense k-qubit gate over 2^kDenseTileLog2-amplitude tiles (staged kernel only)
         if (a.dense.k < kMinDenseK || a.dense.k > kMaxDenseK || a.C + a.j != kDenseTileLog2 || a.code_moves ||
@@ -2772,13 +2875,8 @@ cudaError_t launch_pass(bool f64, const PassArgs &a, int, cudaStream_t s) {
         if (f64) return a.code_moves ? launch_staged_t<double, true>(a, s) : launch_staged_t<double, false>(a, s);
         return a.code_moves ? launch_staged_t<float, true>(a, s) : launch_staged_t<float, false>(a, s);
     }
-    if (f64)
-        return a.code_moves ? launch_pass_t<double, kRegBits, true, 4>(a, s) : launch_pass_t<double, kRegBits, false, 4>(a, s);
-    if (a.code_moves)
-        return a.header_batch == 8 ? launch_pass_t<float, kRegBits, true, 8>(a, s)
-                                   : launch_pass_t<float, kRegBits, true, 4>(a, s);
-    return a.header_batch == 8 ? launch_pass_t<float, kRegBits, false, 8>(a, s)
-                               : launch_pass_t<float, kRegBits, false, 4>(a, s);
+    if (f64) return a.code_moves ? launch_pass_t<double, kRegBits, true>(a, s) : launch_pass_t<double, kRegBits, false>(a, s);
+    return a.code_moves ? launch_pass_t<float, kRegBits, true>(a, s) : launch_pass_t<float, kRegBits, false>(a, s);
 }
 
 cudaError_t launch_perm_pass(const PermPassArgs &a, cudaStream_t s) {
@@ -2790,7 +2888,7 @@ cudaError_t launch_perm_pass(const PermPassArgs &a, cudaStream_t s) {
 template <typename R, int RB, int kC, int kJ>
 static cudaError_t launch_dense_pass_kc(const DensePassArgs &a, cudaStream_t s) {
     const int nb = a.C + a.j;
-    const size_t smem = (size_t)(2 * sizeof(R)) << nb;
+    const size_t smem = tile_bytes<R>(nb);
     auto kern = dense_pass_kernel<R, RB, kC, kJ>;
     cudaError_t e = ensure_dyn_smem(kern, smem);
     if (e != cudaSuccess) return e;
