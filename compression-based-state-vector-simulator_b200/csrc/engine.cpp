@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstring>
 #include <random>
+#include <memory>
 #include <set>
 #include <string>
 #include <thread>
@@ -728,6 +729,89 @@ bool finalize_ops(const std::vector<RawOp> &raw, const std::vector<cplx> &rpool,
     return true;
 }
 
+// Class and place bits of an op code; false for codes that no program holds.
+bool program_op(int code, uint32_t *what) {
+    struct { int base; uint32_t cls; bool pair; } const kinds[] = {
+        {qs::OPC_D2, qs::kProgDiag, false},        {qs::OPC_D2H, qs::kProgHalf, false},
+        {qs::OPC_M2, qs::kProgM2, false},          {qs::OPC_X, qs::kProgX, false},
+        {qs::OPC_D2HP, qs::kProgHalfPending, false}, {qs::OPC_D4, qs::kProgDiag4, true},
+        {qs::OPC_D4H, qs::kProgHalf4, true},       {qs::OPC_M4, qs::kProgM4, true},
+        {qs::OPC_SWAP, qs::kProgSwap, true}};
+    if (code == qs::OPC_SCALAR || code == qs::OPC_ACC) {
+        *what = code == qs::OPC_SCALAR ? qs::kProgScalar : qs::kProgAcc;
+        return true;
+    }
+    for (const auto &k : kinds) {
+        if (code < k.base || code >= k.base + (k.pair ? 32 : 8)) continue;
+        const int a = k.pair ? (code - k.base) >> 3 : 0, b = (code - k.base) & 7;
+        if (a >= qs::kRegBits || b >= qs::kRegBits || (k.pair && a >= b)) return false;
+        // pairs 01, 02, 03, 12, 13, 23
+        const int place = k.pair ? (a == 0 ? b - 1 : a == 1 ? b + 1 : 5) : b;
+        *what = k.cls | (1u << (qs::kProgWhere + place));
+        return true;
+    }
+    return false;
+}
+
+// The program of one pass (internal.h): its sweeps (op ranges relative to
+// ops), ops and fixed matrices in the state's precision.  False when the pass
+// is too long for one.
+bool build_program(const std::vector<qs::Sweep> &sweeps, const qs::ROp *ops, const std::vector<cplx> &pool, bool f64,
+                   qs::PassProgram *out) {
+    std::memset(out, 0, sizeof(*out));
+    if (sweeps.size() > (size_t)qs::kProgSweeps) return false;
+    const size_t entry = f64 ? 16 : 8;
+    size_t used = 0;
+    out->nsweeps = (int32_t)sweeps.size();
+    for (size_t w = 0; w < sweeps.size(); ++w) {
+        const qs::Sweep &sw = sweeps[w];
+        qs::ProgSweep &ps = out->sweeps[w];
+        if (sw.g1 > qs::kProgOps) return false;
+        ps.g0 = sw.g0;
+        ps.g1 = sw.g1;
+        for (int k = 0; k < qs::kRegBits; ++k) ps.sbits[k] = sw.sbits[k];
+        for (int k = sw.g0; k < sw.g1; ++k) {
+            const qs::ROp &o = ops[k];
+            qs::ProgOp &p = out->ops[k];
+            if (!program_op(o.code, &p.what)) return false;
+            p.stride = o.vstride;
+            if (o.code == qs::OPC_SCALAR) ps.scalar = 1;
+            if (o.nsel == 0) {
+                if (used + o.vstride * entry > (size_t)qs::kProgMatBytes) return false;
+                p.mat = (uint32_t)(used / entry);
+                for (int e = 0; e < o.vstride; ++e) {
+                    const cplx c = pool[o.mat + e];
+                    if (f64) {
+                        const double d[2] = {c.real(), c.imag()};
+                        std::memcpy(out->mats + used, d, 16);
+                    } else {
+                        const float d[2] = {(float)c.real(), (float)c.imag()};
+                        std::memcpy(out->mats + used, d, 8);
+                    }
+                    used += entry;
+                }
+                continue;
+            }
+            p.what |= qs::kProgVar;
+            p.mat = o.mat;
+            if (o.sel[0] & qs::kSelRuns) {
+                p.s1 = o.sel[0] & 31u;
+                p.m1 = (1u << o.sel[1]) - 1u;
+                p.s2 = o.sel[2];
+                p.m2 = (1u << o.sel[3]) - 1u;
+                p.l1 = o.sel[1];
+            } else {
+                p.what |= qs::kProgSelList;
+                for (int j = 0; j < 4; ++j) {
+                    p.s1 |= (uint32_t)o.sel[j] << (8 * j);
+                    p.m1 |= (uint32_t)o.sel[4 + j] << (8 * j);
+                }
+            }
+        }
+    }
+    return true;
+}
+
 template <typename Real>
 std::vector<Real> pool_as(const std::vector<cplx> &pool) {
     std::vector<Real> out(2 * pool.size());
@@ -1032,6 +1116,7 @@ struct qs_state {
         int kind;             // 0: tile pass, 1: chunk-header permutation only
         bool code_moves;      // tile pass whose ops only move amplitudes (X / SWAP)
         qs::ChunkPerm perm;   // where the pass stores each chunk
+        std::shared_ptr<const qs::PassProgram> prog;  // the pass's program when it fits one
     };
     qs::Sweep *sweeps_dev = nullptr;
     qs::ROp *ops_dev = nullptr;
@@ -1521,6 +1606,8 @@ static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGat
             printf(" ]\n");
         }
         dp.nsweeps = (uint32_t)swp.size();
+        auto prog = std::make_shared<qs::PassProgram>();
+        if (build_program(swp, ops.data() + op0, pool, h->f64, prog.get())) dp.prog = prog;
         sw.insert(sw.end(), swp.begin(), swp.end());
         out->push_back(dp);
     }
@@ -1905,7 +1992,7 @@ qs_status qs_apply_circuit(qs_state *h) {
         a.stats = stats;
         a.staged = h->staged ? 1 : 0;
         if (e0) CUDA_TRY(h, cudaEventRecord(e0, s));
-        CUDA_TRY(h, qs::launch_pass(h->f64, a, h->tile_log2, s));
+        CUDA_TRY(h, qs::launch_pass(h->f64, a, dp.prog.get(), s));
         if (e1) CUDA_TRY(h, cudaEventRecord(e1, s));
         h->cur = out;
         h->mcur ^= 1;
@@ -2443,7 +2530,7 @@ qs_status qs_apply_dense_gate(qs_state *h, const uint32_t *targets, uint32_t k, 
     a.staged = 1;
     a.dense = dk;
     CUDA_TRY(h, cudaEventRecord(h->ev[0], s));
-    CUDA_TRY(h, qs::launch_pass(h->f64, a, qs::kDenseTileLog2, s));
+    CUDA_TRY(h, qs::launch_pass(h->f64, a, nullptr, s));
     CUDA_TRY(h, cudaEventRecord(h->ev[1], s));
     CUDA_TRY(h, qs::launch_stage_end(db2g, h->group_active, h->nb, h->block_nz, h->block_acc, h->mask,
                                      h->block_bytes, dhist, s));
@@ -2762,7 +2849,7 @@ qs_status qs_apply_diagonal_pauli_sum(qs_state *out, const qs_state *in, const u
     a.diag.terms = dterms;
     a.diag.coefs = dcoef;
     a.diag.nterms = (int)nterms;
-    e = qs::launch_pass(out->f64, a, out->tile_log2, s);
+    e = qs::launch_pass(out->f64, a, nullptr, s);
     // out keeps in's zero-block mask; its block bytes are the new ones
     if (e == cudaSuccess) e = cudaMemcpyAsync(out->mask, in->mask, out->nb, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess)
@@ -3658,8 +3745,8 @@ qs_status qs_dense_apply_gates(qs_dense *h, const qs_gate *gates, size_t count) 
     if ((int)h->n < RB) return qs_dense_apply_gates_pergate(h, gates, count);
     std::vector<uint32_t> ids(count);
     for (size_t i = 0; i < count; ++i) ids[i] = (uint32_t)i;
-    auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, cg, C, jmax, std::min(jmax, 3), C, (int)h->n)
-                                             : plan_passes(ids, cg, C, jmax, std::min(jmax, 3), C, (int)h->n);
+    auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, cg, C, jmax, jmax, C, (int)h->n)
+                                             : plan_passes(ids, cg, C, jmax, jmax, C, (int)h->n);
     std::vector<qs::KGate> kg;
     std::vector<qs::Sweep> sw;
     std::vector<qs::ROp> ops;
@@ -3667,6 +3754,8 @@ qs_status qs_dense_apply_gates(qs_dense *h, const qs_gate *gates, size_t count) 
     std::vector<std::pair<size_t, size_t>> sweep_ranges;
     std::vector<size_t> op_offsets;
     std::vector<std::vector<int>> outers;
+    std::vector<qs::PassProgram> progs;
+    progs.reserve(pl.size());
     for (auto &p : pl) {
         // a tile must hold at least the RB register bits
         std::set<int> t(p.tile.begin(), p.tile.end());
@@ -3686,6 +3775,8 @@ qs_status qs_dense_apply_gates(qs_dense *h, const qs_gate *gates, size_t count) 
         if (!finalize_ops(raw, rpool, C + (int)p.tile.size(), &outer, &ops, &pool))
             return dfail(h, QS_ERR_ARG, "a pass needs more outer selector qubits than the planner allows");
         fuse_half_chains(&ops, op0, swp);
+        progs.emplace_back();
+        if (!build_program(swp, ops.data() + op0, pool, h->f64, &progs.back())) progs.back().nsweeps = -1;
         outers.push_back(outer);
         op_offsets.push_back(op0);
         sweep_ranges.push_back({sw.size(), swp.size()});
@@ -3742,7 +3833,7 @@ qs_status qs_dense_apply_gates(qs_dense *h, const qs_gate *gates, size_t count) 
         for (size_t k = 0; k < outers[pi].size(); ++k) a.outer_q[k] = (int8_t)outers[pi][k];
         a.state = h->state;
         off += p.gates.size();
-        CUDA_TRY(h, qs::launch_dense_pass(h->f64, a, tile_log2, h->stream));
+        CUDA_TRY(h, qs::launch_dense_pass(h->f64, a, progs[pi].nsweeps < 0 ? nullptr : &progs[pi], h->stream));
     }
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     return QS_OK;

@@ -118,6 +118,44 @@ constexpr int kMaxOuterSel = 16;
 static_assert(sizeof(ROp) == 16, "ROp is one 16-byte load");
 static_assert(sizeof(KGate) == 288, "KGate layout");
 
+// A pass's sweeps and ops as a kernel parameter: read through the constant
+// bank with uniform indices, so that the op stream is fetched and branched on
+// by the uniform datapath and a fixed matrix needs no load from memory.  A
+// pass that does not fit runs from global memory (ROp, Sweep) instead.
+//   what      one class bit (kProg*), the register bit or pair it acts on one-hot
+//             from kProgWhere up (bit k; pairs 01, 02, 03, 12, 13, 23), and
+//             kProgVar: its variants lie in the global pool (entry mat +
+//             variant * stride), else its entries lie in mats at entry `mat`
+//   variant   ((W >> s1) & m1) + (((W >> s2) & m2) << l1); with kProgSelList
+//             s1 and m1 hold the selector positions as bytes instead
+// One-hot bits instead of a code: the device tests them one after another, and
+// each test joins two paths only.  A switch over all bodies joined some forty,
+// and the compiler then copied the whole register group (64 registers in
+// double precision) after every op.
+constexpr uint32_t kProgScalar = 1, kProgAcc = 2, kProgHalf = 4, kProgHalfPending = 8, kProgDiag = 16, kProgM2 = 32,
+                   kProgX = 64, kProgHalf4 = 128, kProgDiag4 = 256, kProgM4 = 512, kProgSwap = 1024;
+constexpr uint32_t kProgVar = 1u << 14, kProgSelList = 1u << 15;
+constexpr int kProgWhere = 16;
+constexpr int kProgOps = 80, kProgSweeps = 16, kProgMatBytes = 6144;
+struct ProgOp {
+    uint32_t what, mat, stride, s1, m1, s2, m2, l1;
+};
+struct ProgSweep {
+    int32_t g0, g1;
+    int32_t sbits[kRegBits];
+    int32_t scalar;             // some op is OPC_SCALAR: the group's factor has to be applied
+    int32_t pad;
+};
+struct PassProgram {
+    int32_t nsweeps;
+    int32_t pad[3];
+    ProgSweep sweeps[kProgSweeps];
+    ProgOp ops[kProgOps];
+    // complex entries of the state's precision; one op's worth of slack, since
+    // the device reads four entries of every fixed op
+    alignas(16) unsigned char mats[kProgMatBytes + 64];
+};
+
 struct CodecParams {
     int32_t m;      // mantissa bits kept (relative step 2^-m)
     int32_t L;      // absolute step 2^-L in the linear region
@@ -369,11 +407,12 @@ cudaError_t launch_dense_pauli_sum(bool f64, const void *in, void *out, int n, c
 cudaError_t launch_expect(bool f64, const ExpectArgs &a, cudaStream_t stream);
 cudaError_t launch_dense_expect(bool f64, const void *state, int n, const PauliTerm *terms, int nterms, double *out,
                                 cudaStream_t stream);
-cudaError_t launch_pass(bool f64, const PassArgs &a, int tile_log2, cudaStream_t stream);
+// prog: the pass's program when it fits one, else NULL.
+cudaError_t launch_pass(bool f64, const PassArgs &a, const PassProgram *prog, cudaStream_t stream);
 // Shared memory of one staged_pass_kernel CTA for tiles of 2^(C+j) amplitudes.
 size_t staged_pass_smem_bytes(bool f64, int C, int j, uint32_t nblocks);
 cudaError_t launch_perm_pass(const PermPassArgs &a, cudaStream_t stream);
-cudaError_t launch_dense_pass(bool f64, const DensePassArgs &a, int tile_log2, cudaStream_t stream);
+cudaError_t launch_dense_pass(bool f64, const DensePassArgs &a, const PassProgram *prog, cudaStream_t stream);
 cudaError_t launch_pergate(bool f64, void *state, int n, const KGate *gate_dev, cudaStream_t stream);
 
 cudaError_t launch_stage_begin(const uint32_t *block_to_group, const uint8_t *mask, uint32_t nb,

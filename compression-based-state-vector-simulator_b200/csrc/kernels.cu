@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "codec.cuh"
 #include "internal.h"
@@ -343,6 +344,156 @@ __device__ __forceinline__ void tile_sweeps_body(typename Cplx<R>::T *tile, int 
         __syncthreads();
     }
 }
+// One op of a program.  Its class and place are uniform, so each branch is.
+template <int RB, typename T>
+__device__ __forceinline__ void apply_prog_op(T (&v)[1 << RB], T &z, T &zh, const PassProgram &pr, int k,
+                                              const T *__restrict__ pool, uint32_t W) {
+    constexpr int NS = 1 << RB;
+    static_assert(RB == 4, "the place bits of ProgOp name four register bits");
+    const ProgOp &o = pr.ops[k];
+    const T *const mats = reinterpret_cast<const T *>(pr.mats);
+    const uint32_t what = o.what;
+    const uint32_t at = what >> kProgWhere;
+    T e0, e1, e2, e3;
+    if (what & kProgVar) {
+        uint32_t var;
+        if (what & kProgSelList) {
+            var = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                var |= ((W >> ((o.s1 >> (8 * j)) & 31u)) & 1u) << j;
+                var |= ((W >> ((o.m1 >> (8 * j)) & 31u)) & 1u) << (4 + j);
+            }
+        } else {
+            var = ((W >> o.s1) & o.m1) + (((W >> o.s2) & o.m2) << o.l1);
+        }
+        const T *const p = pool + o.mat + var * o.stride;
+        e0 = p[0];
+        if (o.stride > 1) e1 = p[1];
+        if (o.stride > 2) {
+            e2 = p[2];
+            e3 = p[3];
+        }
+    } else {
+        e0 = mats[o.mat];
+        e1 = mats[o.mat + 1];
+        e2 = mats[o.mat + 2];
+        e3 = mats[o.mat + 3];
+    }
+    if (what & (kProgScalar | kProgAcc | kProgHalf | kProgHalfPending)) {
+        if (what & kProgScalar) z = cmul(z, e0);
+        if (what & kProgAcc) zh = cmul(zh, e0);
+        if (what & kProgHalfPending) {
+            e0 = cmul(zh, e0);
+            zh = c_one<T>();
+        }
+        if (at & 1) r_half2<NS, 0>(v, e0);
+        if (at & 2) r_half2<NS, 1>(v, e0);
+        if (at & 4) r_half2<NS, 2>(v, e0);
+        if (at & 8) r_half2<NS, 3>(v, e0);
+        return;
+    }
+    if (what & kProgM4) {
+        if (at & 1) r_4x4<NS, 0, 1>(v, mats + o.mat);
+        if (at & 2) r_4x4<NS, 0, 2>(v, mats + o.mat);
+        if (at & 4) r_4x4<NS, 0, 3>(v, mats + o.mat);
+        if (at & 8) r_4x4<NS, 1, 2>(v, mats + o.mat);
+        if (at & 16) r_4x4<NS, 1, 3>(v, mats + o.mat);
+        if (at & 32) r_4x4<NS, 2, 3>(v, mats + o.mat);
+        return;
+    }
+    if (what & kProgM2) {
+        if (at & 1) r_2x2<NS, 0>(v, e0, e1, e2, e3);
+        if (at & 2) r_2x2<NS, 1>(v, e0, e1, e2, e3);
+        if (at & 4) r_2x2<NS, 2>(v, e0, e1, e2, e3);
+        if (at & 8) r_2x2<NS, 3>(v, e0, e1, e2, e3);
+        return;
+    }
+    if (what & kProgHalf4) {
+        if (at & 1) r_half4<NS, 0, 1>(v, e0, e1, e2);
+        if (at & 2) r_half4<NS, 0, 2>(v, e0, e1, e2);
+        if (at & 4) r_half4<NS, 0, 3>(v, e0, e1, e2);
+        if (at & 8) r_half4<NS, 1, 2>(v, e0, e1, e2);
+        if (at & 16) r_half4<NS, 1, 3>(v, e0, e1, e2);
+        if (at & 32) r_half4<NS, 2, 3>(v, e0, e1, e2);
+        return;
+    }
+    if (what & kProgDiag) {
+        if (at & 1) r_diag2<NS, 0>(v, e0, e1);
+        if (at & 2) r_diag2<NS, 1>(v, e0, e1);
+        if (at & 4) r_diag2<NS, 2>(v, e0, e1);
+        if (at & 8) r_diag2<NS, 3>(v, e0, e1);
+        return;
+    }
+    if (what & kProgDiag4) {
+        if (at & 1) r_diag4<NS, 0, 1>(v, e0, e1, e2, e3);
+        if (at & 2) r_diag4<NS, 0, 2>(v, e0, e1, e2, e3);
+        if (at & 4) r_diag4<NS, 0, 3>(v, e0, e1, e2, e3);
+        if (at & 8) r_diag4<NS, 1, 2>(v, e0, e1, e2, e3);
+        if (at & 16) r_diag4<NS, 1, 3>(v, e0, e1, e2, e3);
+        if (at & 32) r_diag4<NS, 2, 3>(v, e0, e1, e2, e3);
+        return;
+    }
+    if (what & kProgX) {
+        if (at & 1) r_x<NS, 0>(v);
+        if (at & 2) r_x<NS, 1>(v);
+        if (at & 4) r_x<NS, 2>(v);
+        if (at & 8) r_x<NS, 3>(v);
+    } else {  // kProgSwap
+        if (at & 1) r_swap<NS, 0, 1>(v);
+        if (at & 2) r_swap<NS, 0, 2>(v);
+        if (at & 4) r_swap<NS, 0, 3>(v);
+        if (at & 8) r_swap<NS, 1, 2>(v);
+        if (at & 16) r_swap<NS, 1, 3>(v);
+        if (at & 32) r_swap<NS, 2, 3>(v);
+    }
+}
+
+// The sweeps of a pass whose program is a kernel parameter.
+template <typename R, int RB>
+__device__ __forceinline__ void tile_sweeps_prog(typename Cplx<R>::T *tile, int nb, const PassProgram &pr,
+                                                 const typename Cplx<R>::T *__restrict__ pool, uint32_t ow) {
+    using T = typename Cplx<R>::T;
+    constexpr int NS = 1 << RB;
+    static_assert(RB == kRegBits, "ProgSweep holds kRegBits bits");
+    const int groups = 1 << (nb - RB);
+    const uint32_t wo = ow << nb;
+    for (int w = 0; w < pr.nsweeps; ++w) {
+        const ProgSweep &sw = pr.sweeps[w];
+        int olo[4], ohi[4];
+        {
+            const int p0 = pos<R>(1 << sw.sbits[0]), p1 = pos<R>(1 << sw.sbits[1]);
+            const int p2 = pos<R>(1 << sw.sbits[2]), p3 = pos<R>(1 << sw.sbits[3]);
+            olo[0] = 0, olo[1] = p0, olo[2] = p1, olo[3] = p0 + p1;
+            ohi[0] = 0, ohi[1] = p2, ohi[2] = p3, ohi[3] = p2 + p3;
+        }
+        for (int grp = threadIdx.x; grp < groups; grp += blockDim.x) {
+            int base = grp;
+#pragma unroll
+            for (int k = 0; k < RB; ++k) {
+                const int t = sw.sbits[k];
+                base = ((base >> t) << (t + 1)) | (base & ((1 << t) - 1));
+            }
+            const uint32_t W = (uint32_t)base | wo;
+            T *const g = tile + pos<R>(base);
+            T v[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) v[s] = g[olo[s & 3] + ohi[s >> 2]];
+            T z = c_one<T>(), zh = c_one<T>();
+            for (int k = sw.g0; k < sw.g1; ++k) apply_prog_op<RB>(v, z, zh, pr, k, pool, W);
+            if (sw.scalar) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) v[s] = cmul(z, v[s]);
+            }
+#pragma unroll
+            for (int s = 0; s < NS; ++s) g[olo[s & 3] + ohi[s >> 2]] = v[s];
+        }
+        __syncthreads();
+    }
+}
+
+struct NoProgram {};
+
 template <typename R, int RB>
 __device__ __noinline__ void tile_sweeps_call(typename Cplx<R>::T *tile, int nb, const Sweep *__restrict__ sweeps,
                             int nsweeps, const ROp *__restrict__ ops, const typename Cplx<R>::T *__restrict__ pool,
@@ -397,6 +548,16 @@ __device__ __forceinline__ void issue_payload(const uint32_t *__restrict__ arena
     for (int off = lane * 16; off < rows * 128; off += 32 * 16)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sdst + off), "l"(gsrc + off) : "memory");
     asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// One element (8 or 16 bytes) copied into shared memory without a register.
+template <int kBytes>
+__device__ __forceinline__ void cp_async_elem(void *dst, const void *src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (kBytes == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
 
 template <int N>
@@ -777,8 +938,11 @@ __device__ void tile_diag_sum(typename Cplx<R>::T *tile, int nb, const DiagSum &
 // only around the sweeps: between a tile's encode and the next one's decode
 // its warps run apart.  All payloads of a warp's chunks are copied at once,
 // each into its chunk's own tile region (no staging buffer).
-template <typename R, int RB, bool kCodes, int kC, int kJ>
-__global__ void __launch_bounds__(kSweepThreads, 3) pass_kernel(const PassArgs a) {
+// Prog: PassProgram (the default geometry), or NoProgram: the ops are read
+// from global memory.
+template <typename R, int RB, bool kCodes, int kC, int kJ, typename Prog>
+__global__ void __launch_bounds__(kSweepThreads, 3) pass_kernel(const __grid_constant__ PassArgs a,
+                                                                const __grid_constant__ Prog prog) {
     using T = typename Cplx<R>::T;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int32_t s_tq[kMaxTileQubits];
@@ -844,8 +1008,11 @@ __global__ void __launch_bounds__(kSweepThreads, 3) pass_kernel(const PassArgs a
         __syncthreads();
 
         // ---- gates
-        tile_sweeps<R, RB>(tile, nb, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool),
-                           outer_word(chunk_base << C, s_oq, a.nouter));
+        const uint32_t ow = outer_word(chunk_base << C, s_oq, a.nouter);
+        if constexpr (std::is_same_v<Prog, PassProgram>)
+            tile_sweeps_prog<R, RB>(tile, nb, prog, reinterpret_cast<const T *>(a.pool), ow);
+        else
+            tile_sweeps<R, RB>(tile, nb, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool), ow);
         if constexpr (!kCodes) {
             if (a.diag.nterms)
                 tile_diag_sum<R>(tile, nb, a.diag, chunk_base << C, reinterpret_cast<double *>(s_out + nchunks));
@@ -1593,8 +1760,9 @@ __global__ void perm_pass_kernel(const PermPassArgs a) {
 // ------------------------------------------------------------ dense pass
 // kC, kJ: the chunk and tile-qubit counts as compile-time constants (0 = read
 // them from the launch arguments).
-template <typename R, int RB, int kC, int kJ>
-__global__ void __launch_bounds__(kSweepThreads, 3) dense_pass_kernel(const DensePassArgs a) {
+template <typename R, int RB, int kC, int kJ, typename Prog>
+__global__ void __launch_bounds__(kSweepThreads, 3) dense_pass_kernel(const __grid_constant__ DensePassArgs a,
+                                                                      const __grid_constant__ Prog prog) {
     using T = typename Cplx<R>::T;
     extern __shared__ __align__(16) unsigned char smem[];
     T *tile = reinterpret_cast<T *>(smem);
@@ -1602,24 +1770,38 @@ __global__ void __launch_bounds__(kSweepThreads, 3) dense_pass_kernel(const Dens
     const int C = kC ? kC : a.C, j = kJ ? kJ : a.j, nb = C + j;
     const int size = 1 << nb;
     const int cmask = (1 << C) - 1;
+    // amplitude offset of each of the tile's 2^j chunks, the same for every tile
+    uint64_t *s_off = reinterpret_cast<uint64_t *>(smem + tile_bytes<R>(nb));
     __shared__ int32_t s_tq[kMaxTileQubits];
     __shared__ int8_t s_oq[kMaxOuterSel];
     if (threadIdx.x < kMaxTileQubits) s_tq[threadIdx.x] = a.tq[threadIdx.x];
     if (threadIdx.x < kMaxOuterSel) s_oq[threadIdx.x] = a.outer_q[threadIdx.x];
     __syncthreads();
+    for (int c = threadIdx.x; c < (1 << j); c += blockDim.x) s_off[c] = deposit_bits((uint32_t)c, s_tq, j) << C;
+    __syncthreads();
     for (uint64_t tile_id = blockIdx.x; tile_id < a.n_tiles; tile_id += gridDim.x) {
         const uint64_t chunk_base = insert_zero_bits(tile_id, s_tq, j);
-        for (int e = threadIdx.x; e < size; e += blockDim.x) {
-            const uint64_t amp = ((chunk_base | deposit_bits((uint32_t)(e >> C), s_tq, j)) << C) | (uint64_t)(e & cmask);
-            tile[pos<R>(e)] = st[amp];
-        }
+        T *const st0 = st + (chunk_base << C);
+        // every load of the tile in flight at once, straight into shared memory
+#pragma unroll 4
+        for (int e = threadIdx.x; e < size; e += kSweepThreads)
+            cp_async_elem<sizeof(T)>(&tile[pos<R>(e)], &st0[s_off[e >> C] + (e & cmask)]);
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
-        tile_sweeps<R, RB>(tile, nb, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool),
-                           outer_word(chunk_base << C, s_oq, a.nouter));
-        for (int e = threadIdx.x; e < size; e += blockDim.x) {
-            const uint64_t amp = ((chunk_base | deposit_bits((uint32_t)(e >> C), s_tq, j)) << C) | (uint64_t)(e & cmask);
-            st[amp] = tile[pos<R>(e)];
+        // the CTA's next tile starts its way into L2 while this one is worked on
+        if (tile_id + gridDim.x < a.n_tiles) {
+            const T *const nx = st + (insert_zero_bits(tile_id + gridDim.x, s_tq, j) << C);
+            constexpr int kLine = 128 / sizeof(T);
+            for (int e = threadIdx.x * kLine; e < size; e += kSweepThreads * kLine)
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx + s_off[e >> C] + (e & cmask)));
         }
+        const uint32_t ow = outer_word(chunk_base << C, s_oq, a.nouter);
+        if constexpr (std::is_same_v<Prog, PassProgram>)
+            tile_sweeps_prog<R, RB>(tile, nb, prog, reinterpret_cast<const T *>(a.pool), ow);
+        else
+            tile_sweeps<R, RB>(tile, nb, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool), ow);
+#pragma unroll 8
+        for (int e = threadIdx.x; e < size; e += kSweepThreads) st0[s_off[e >> C] + (e & cmask)] = tile[pos<R>(e)];
         __syncthreads();
     }
 }
@@ -2789,14 +2971,14 @@ int sm_count() {
     return g_sm_count;
 }
 
-template <typename R, int RB, bool kCodes, int kC, int kJ>
-static cudaError_t launch_pass_kc(const PassArgs &a, cudaStream_t s) {
+template <typename R, int RB, bool kCodes, int kC, int kJ, typename Prog>
+static cudaError_t launch_pass_kc(const PassArgs &a, const Prog &prog, cudaStream_t s) {
     const int nb = a.C + a.j;
     const size_t smem = pass_smem_bytes(sizeof(R) == 8, nb, a.j, a.diag.nterms);
-    cudaError_t e = ensure_dyn_smem(pass_kernel<R, RB, kCodes, kC, kJ>, smem);
+    cudaError_t e = ensure_dyn_smem(pass_kernel<R, RB, kCodes, kC, kJ, Prog>, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<R, RB, kCodes, kC, kJ>, kSweepThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<R, RB, kCodes, kC, kJ, Prog>, kSweepThreads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     uint64_t grid = (uint64_t)per_sm * sm_count();
@@ -2808,7 +2990,7 @@ static cudaError_t launch_pass_kc(const PassArgs &a, cudaStream_t s) {
     const char *env = std::getenv("QOMPSIM_SLAB_BYTES");
     const uint64_t slab = env ? (uint64_t)std::strtoull(env, nullptr, 10) : (uint64_t)kArenaSlabBytes;
     b.slab = (slab && a.capacity / grid >= 8 * slab) ? (slab + 127) / 128 * 128 : 0;
-    pass_kernel<R, RB, kCodes, kC, kJ><<<(unsigned)grid, kSweepThreads, smem, s>>>(b);
+    pass_kernel<R, RB, kCodes, kC, kJ, Prog><<<(unsigned)grid, kSweepThreads, smem, s>>>(b, prog);
     return cudaGetLastError();
 }
 
@@ -2817,12 +2999,15 @@ static cudaError_t launch_pass_kc(const PassArgs &a, cudaStream_t s) {
 // above the chunk) are compile-time constants of their instantiation: the
 // per-lane counts, chunk and group counts, offsets and swizzle mask then fold
 // into the code (measured 12-19 % faster than reading them from the args).
+// These instantiations read their ops from a program; longer op lists run from
+// global memory in the run-time geometry.
 template <typename R, int RB, bool kCodes>
-static cudaError_t launch_pass_t(const PassArgs &a, cudaStream_t s) {
+static cudaError_t launch_pass_t(const PassArgs &a, const PassProgram *prog, cudaStream_t s) {
     constexpr int J = sizeof(R) == 8 ? 4 : 5;
-    if (a.C == kMaxChunkLog2 && a.j == J) return launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, J>(a, s);
-    return a.C == kMaxChunkLog2 ? launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, 0>(a, s)
-                                : launch_pass_kc<R, RB, kCodes, 0, 0>(a, s);
+    if (a.C == kMaxChunkLog2 && a.j == J && prog)
+        return launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, J, PassProgram>(a, *prog, s);
+    return a.C == kMaxChunkLog2 ? launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, 0, NoProgram>(a, NoProgram{}, s)
+                                : launch_pass_kc<R, RB, kCodes, 0, 0, NoProgram>(a, NoProgram{}, s);
 }
 
 template <typename R, bool kCodes, bool kDense, int kC, int kJ>
@@ -2859,7 +3044,7 @@ static cudaError_t launch_staged_t(const PassArgs &a, cudaStream_t s) {
     return launch_staged_kc<R, kCodes, kDense, 0, 0>(a, s);
 }
 
-cudaError_t launch_pass(bool f64, const PassArgs &a, int, cudaStream_t s) {
+cudaError_t launch_pass(bool f64, const PassArgs &a, const PassProgram *prog, cudaStream_t s) {
     if (a.rb != kRegBits || a.C + a.j < kRegBits || a.diag.nterms > kMaxDiagTerms) return cudaErrorInvalidValue;
     if (a.code_moves && a.diag.nterms) return cudaErrorInvalidValue;
     if (a.dense.k) {
@@ -2875,8 +3060,11 @@ cudaError_t launch_pass(bool f64, const PassArgs &a, int, cudaStream_t s) {
         if (f64) return a.code_moves ? launch_staged_t<double, true>(a, s) : launch_staged_t<double, false>(a, s);
         return a.code_moves ? launch_staged_t<float, true>(a, s) : launch_staged_t<float, false>(a, s);
     }
-    if (f64) return a.code_moves ? launch_pass_t<double, kRegBits, true>(a, s) : launch_pass_t<double, kRegBits, false>(a, s);
-    return a.code_moves ? launch_pass_t<float, kRegBits, true>(a, s) : launch_pass_t<float, kRegBits, false>(a, s);
+    if (f64)
+        return a.code_moves ? launch_pass_t<double, kRegBits, true>(a, prog, s)
+                            : launch_pass_t<double, kRegBits, false>(a, prog, s);
+    return a.code_moves ? launch_pass_t<float, kRegBits, true>(a, prog, s)
+                        : launch_pass_t<float, kRegBits, false>(a, prog, s);
 }
 
 cudaError_t launch_perm_pass(const PermPassArgs &a, cudaStream_t s) {
@@ -2885,11 +3073,11 @@ cudaError_t launch_perm_pass(const PermPassArgs &a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <typename R, int RB, int kC, int kJ>
-static cudaError_t launch_dense_pass_kc(const DensePassArgs &a, cudaStream_t s) {
+template <typename R, int RB, int kC, int kJ, typename Prog>
+static cudaError_t launch_dense_pass_kc(const DensePassArgs &a, const Prog &prog, cudaStream_t s) {
     const int nb = a.C + a.j;
-    const size_t smem = tile_bytes<R>(nb);
-    auto kern = dense_pass_kernel<R, RB, kC, kJ>;
+    const size_t smem = tile_bytes<R>(nb) + ((size_t)8 << a.j);
+    auto kern = dense_pass_kernel<R, RB, kC, kJ, Prog>;
     cudaError_t e = ensure_dyn_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -2899,22 +3087,22 @@ static cudaError_t launch_dense_pass_kc(const DensePassArgs &a, cudaStream_t s) 
     uint64_t grid = (uint64_t)per_sm * sm_count();
     if (grid > a.n_tiles) grid = a.n_tiles;
     if (grid == 0) grid = 1;
-    kern<<<(unsigned)grid, kSweepThreads, smem, s>>>(a);
+    kern<<<(unsigned)grid, kSweepThreads, smem, s>>>(a, prog);
     return cudaGetLastError();
 }
 
 // The uncompressed fused path's default geometry: 2^5-amplitude chunks and
 // tiles of 2^12 (complex128) or 2^13 (complex64) amplitudes.
 template <typename R, int RB>
-static cudaError_t launch_dense_pass_t(const DensePassArgs &a, cudaStream_t s) {
+static cudaError_t launch_dense_pass_t(const DensePassArgs &a, const PassProgram *prog, cudaStream_t s) {
     constexpr int kDC = 5, kDJ = sizeof(R) == 8 ? 7 : 8;
-    if (a.C == kDC && a.j == kDJ) return launch_dense_pass_kc<R, RB, kDC, kDJ>(a, s);
-    return launch_dense_pass_kc<R, RB, 0, 0>(a, s);
+    if (a.C == kDC && a.j == kDJ && prog) return launch_dense_pass_kc<R, RB, kDC, kDJ, PassProgram>(a, *prog, s);
+    return launch_dense_pass_kc<R, RB, 0, 0, NoProgram>(a, NoProgram{}, s);
 }
 
-cudaError_t launch_dense_pass(bool f64, const DensePassArgs &a, int, cudaStream_t s) {
+cudaError_t launch_dense_pass(bool f64, const DensePassArgs &a, const PassProgram *prog, cudaStream_t s) {
     if (a.rb != kRegBits || a.C + a.j < kRegBits) return cudaErrorInvalidValue;
-    return f64 ? launch_dense_pass_t<double, kRegBits>(a, s) : launch_dense_pass_t<float, kRegBits>(a, s);
+    return f64 ? launch_dense_pass_t<double, kRegBits>(a, prog, s) : launch_dense_pass_t<float, kRegBits>(a, prog, s);
 }
 
 cudaError_t launch_pergate(bool f64, void *state, int n, const KGate *g, cudaStream_t s) {
