@@ -66,7 +66,8 @@ struct Sweep {
     int32_t g0, g1;
     int32_t sbits[6];
 };
-// Threads of the fused pass kernels (compressed and dense): 4 warps per CTA.
+// Threads of the uncompressed fused pass kernel: 4 warps per CTA, three CTAs per
+// SM.  (pass_kernel: PassShape in kernels.cu.)
 constexpr int kSweepThreads = 128;
 
 // One register op (host-built, 16 bytes).  `code` names the action and the

@@ -938,11 +938,22 @@ __device__ void tile_diag_sum(typename Cplx<R>::T *tile, int nb, const DiagSum &
 // only around the sweeps: between a tile's encode and the next one's decode
 // its warps run apart.  All payloads of a warp's chunks are copied at once,
 // each into its chunk's own tile region (no staging buffer).
+// Threads of a CTA and CTAs per SM.  complex64 fits 16 warps an SM without
+// spilling (110 registers): QFT n=25 in-block pass 642 -> 567 us, brickwork
+// single-sweep pass 382 -> 335 us against 12 warps.  complex128 spills at 128
+// registers and gains nothing (640 / 620 us, 184 / 188 us); nor does the
+// uncompressed pass (complex64 375 -> 405 us, complex128 762 -> 789 us).
+template <typename R>
+struct PassShape {
+    static constexpr int kThreads = sizeof(R) == 8 ? 128 : 256;
+    static constexpr int kCtas = sizeof(R) == 8 ? 3 : 2;
+};
+
 // Prog: PassProgram (the default geometry), or NoProgram: the ops are read
 // from global memory.
 template <typename R, int RB, bool kCodes, int kC, int kJ, typename Prog>
-__global__ void __launch_bounds__(kSweepThreads, 3) pass_kernel(const __grid_constant__ PassArgs a,
-                                                                const __grid_constant__ Prog prog) {
+__global__ void __launch_bounds__(PassShape<R>::kThreads, PassShape<R>::kCtas)
+    pass_kernel(const __grid_constant__ PassArgs a, const __grid_constant__ Prog prog) {
     using T = typename Cplx<R>::T;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int32_t s_tq[kMaxTileQubits];
@@ -973,7 +984,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) pass_kernel(const __grid_con
         s_out[c] = move_perm(a.perm, s_in[c]);
     }
     __syncthreads();
-    const unsigned long long slab = a.slab / (kSweepThreads / 32) / 128 * 128;  // per warp
+    const unsigned long long slab = a.slab / (PassShape<R>::kThreads / 32) / 128 * 128;  // per warp
 
     WarpArena wa;
     unsigned long long rd = 0, wr = 0, ntiles = 0;
@@ -2978,7 +2989,8 @@ static cudaError_t launch_pass_kc(const PassArgs &a, const Prog &prog, cudaStrea
     cudaError_t e = ensure_dyn_smem(pass_kernel<R, RB, kCodes, kC, kJ, Prog>, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<R, RB, kCodes, kC, kJ, Prog>, kSweepThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<R, RB, kCodes, kC, kJ, Prog>,
+                                                      PassShape<R>::kThreads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     uint64_t grid = (uint64_t)per_sm * sm_count();
@@ -2990,7 +3002,7 @@ static cudaError_t launch_pass_kc(const PassArgs &a, const Prog &prog, cudaStrea
     const char *env = std::getenv("QOMPSIM_SLAB_BYTES");
     const uint64_t slab = env ? (uint64_t)std::strtoull(env, nullptr, 10) : (uint64_t)kArenaSlabBytes;
     b.slab = (slab && a.capacity / grid >= 8 * slab) ? (slab + 127) / 128 * 128 : 0;
-    pass_kernel<R, RB, kCodes, kC, kJ, Prog><<<(unsigned)grid, kSweepThreads, smem, s>>>(b, prog);
+    pass_kernel<R, RB, kCodes, kC, kJ, Prog><<<(unsigned)grid, PassShape<R>::kThreads, smem, s>>>(b, prog);
     return cudaGetLastError();
 }
 
