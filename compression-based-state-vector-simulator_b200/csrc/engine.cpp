@@ -2211,6 +2211,35 @@ qs_status qs_norm_squared(qs_state *h, double *out) {
     return QS_OK;
 }
 
+// Whether [p, p + bytes) lies in one device allocation of the current GPU and
+// p is aligned for doubles, so that a kernel may write it.  (A range that
+// reaches past its allocation is left to the copies, which refuse it.)
+static bool device_range(const void *p, uint64_t bytes) {
+    cudaPointerAttributes at{};
+    int dev = -1;
+    if ((reinterpret_cast<size_t>(p) & 7) != 0 || cudaPointerGetAttributes(&at, p) != cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (at.type != cudaMemoryTypeDevice || at.device != dev) return false;
+    using RangeFn = int (*)(unsigned long long *, size_t *, unsigned long long);
+    static const RangeFn range = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult r = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<RangeFn>(f);
+    }();
+    unsigned long long base = 0;
+    size_t size = 0;
+    const unsigned long long addr = reinterpret_cast<unsigned long long>(p);
+    return range && range(&base, &size, addr) == 0 && addr >= base && bytes <= size && addr - base <= size - bytes;
+}
+
 qs_status qs_get_vector(qs_state *h, double *out, int renormalize) {
     if (!h) return fail(nullptr, QS_ERR_ARG, "NULL handle");
     return qs_get_amplitudes(h, 0, uint64_t(1) << h->n, out, renormalize);
@@ -2232,6 +2261,14 @@ qs_status qs_get_amplitudes(qs_state *h, uint64_t first, uint64_t count, double 
     }
     const uint64_t cfirst = first / chunk_amps, ccount = count / chunk_amps;
     if (!ccount) return QS_OK;
+    // device memory of this GPU is written by the decode itself: no staging
+    // buffer, copy or synchronisation per slab
+    if (device_range(out, count * 2 * sizeof(double))) {
+        CUDA_TRY(h, qs::launch_readout(h->f64, h->meta[h->mcur], h->arena[h->cur], h->mask, (int)h->B, (int)h->C,
+                                       h->codec, cfirst, ccount, out, scale, h->stream));
+        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+        return QS_OK;
+    }
     const uint64_t slab_chunks = std::max<uint64_t>(1, (uint64_t(1) << 24) / chunk_amps);
     double *dbuf = nullptr;
     const uint64_t nslab = std::min<uint64_t>(slab_chunks, ccount);

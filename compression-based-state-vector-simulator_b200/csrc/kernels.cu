@@ -708,19 +708,18 @@ __device__ __forceinline__ uint32_t *chunk_stage(typename Cplx<R>::T *tile, int 
     return reinterpret_cast<uint32_t *>((p + 15) & ~size_t(15));
 }
 
-// Per-warp decode of a chunk whose payload lies in the chunk's own tile region
-// (`src`, payload words; at most as many bytes as the values need): every lane
-// extracts its codes into registers, then the warp overwrites the region with
-// the values.  A chunk whose codes all lie in the linear region (its base and
-// width say so) skips the log region's half of the dequantisation.
-template <typename R, bool kCodes, int kPL>
-__device__ __forceinline__ void unpack_in_place(const ChunkMeta md, int per_lane, CodecParams p,
-                                                typename Cplx<R>::T *chunk_elem0, const uint32_t *src, int lane) {
+// Per-warp decode of a chunk whose payload words are in shared memory at src:
+// every lane extracts its codes into registers, then hands its amplitudes to
+// f(i, value), i = 0, 1, ... for amplitudes k + 16 (i0 + i).  src may be the
+// memory that f writes (kInPlace).  A chunk whose codes all lie in the linear
+// region (its base and width say so) skips the log region's half of the
+// dequantisation.
+template <typename R, bool kCodes, int kPL, bool kInPlace, typename F>
+__device__ __forceinline__ void decode_pairs(const ChunkMeta md, int per_lane, CodecParams p, const uint32_t *src,
+                                             int lane, F f) {
     using T = typename Cplx<R>::T;
     const PairLanes<kPL> pl(per_lane, lane);
     constexpr int H = PairLanes<kPL>::H;
-    T *const dst = chunk_elem0 + pos<R>(16 * pl.i0) + pos<R>(pl.k);
-    constexpr int kStep = 16 + (16 >> Layout<R>::S1);
     // a width above 32 never comes from a pass or a checked import (unpack_chunk)
     const uint32_t w = md.width > 32 ? 32u : md.width;
     if (w == 0) {
@@ -728,7 +727,7 @@ __device__ __forceinline__ void unpack_in_place(const ChunkMeta md, int per_lane
         v.x = v.y = kCodes ? code_as_value(md.base, R()) : dequantize_hot(md.base, p, R());
 #pragma unroll
         for (int i = 0; i < H; ++i)
-            if (i < pl.n) dst[i * kStep] = v;
+            if (i < pl.n) f(i, v);
         return;
     }
     const uint32_t mask = (w >= 32) ? 0xffffffffu : ((1u << w) - 1u);
@@ -745,7 +744,7 @@ __device__ __forceinline__ void unpack_in_place(const ChunkMeta md, int per_lane
             bit += w;
         }
     }
-    __syncwarp();
+    if (kInPlace) __syncwarp();
     if (!kCodes && chunk_is_linear(md.base, w, p, R())) {
 #pragma unroll
         for (int i = 0; i < H; ++i)
@@ -753,7 +752,7 @@ __device__ __forceinline__ void unpack_in_place(const ChunkMeta md, int per_lane
                 T v;
                 v.x = dequantize_linear(q0[i], p, R());
                 v.y = dequantize_linear(q1[i], p, R());
-                dst[i * kStep] = v;
+                f(i, v);
             }
     } else {
 #pragma unroll
@@ -762,9 +761,56 @@ __device__ __forceinline__ void unpack_in_place(const ChunkMeta md, int per_lane
                 T v;
                 v.x = kCodes ? code_as_value(q0[i], R()) : dequantize_hot(q0[i], p, R());
                 v.y = kCodes ? code_as_value(q1[i], R()) : dequantize_hot(q1[i], p, R());
-                dst[i * kStep] = v;
+                f(i, v);
             }
     }
+}
+
+// The chunk starting at tile element chunk_elem0, decoded from the payload
+// words at src inside its own tile region (at most as many bytes as the values).
+template <typename R, bool kCodes, int kPL>
+__device__ __forceinline__ void unpack_in_place(const ChunkMeta md, int per_lane, CodecParams p,
+                                                typename Cplx<R>::T *chunk_elem0, const uint32_t *src, int lane) {
+    using T = typename Cplx<R>::T;
+    const PairLanes<kPL> pl(per_lane, lane);
+    T *const dst = chunk_elem0 + pos<R>(16 * pl.i0) + pos<R>(pl.k);
+    constexpr int kStep = 16 + (16 >> Layout<R>::S1);
+    decode_pairs<R, kCodes, kPL, true>(md, per_lane, p, src, lane, [&](int i, T v) { dst[i * kStep] = v; });
+}
+
+// A warp's chunks gw, gw + nw, ... of [chunk0, chunk0 + nchunks) in turn:
+// fn(k, header, payload words in shared memory), the next chunk's payload
+// copied meanwhile and the header of the one after loaded.  Chunks of unstored
+// blocks come as zero headers.  stage: 2 x kStageWords words per warp.
+template <typename F>
+__device__ __forceinline__ void stream_chunks(const ChunkMeta *__restrict__ meta, const uint32_t *__restrict__ arena,
+                                              const uint8_t *__restrict__ mask, int B, int C, uint64_t chunk0,
+                                              uint64_t nchunks, uint32_t *stage, int lane, F fn) {
+    const int per_lane = (2 << C) >> 5;
+    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    auto header = [&](uint64_t k) {
+        ChunkMeta md{0, 0, 0};
+        if (k < nchunks && mask[(chunk0 + k) >> (B - C)]) md = meta[chunk0 + k];
+        return md;
+    };
+    if (gw >= nchunks) return;
+    ChunkMeta cur = header(gw);
+    issue_payload(arena, cur, per_lane, stage, lane);
+    ChunkMeta next = header(gw + nw);
+    int b = 0;
+    for (uint64_t k = gw; k < nchunks; k += nw) {
+        issue_payload(arena, next, per_lane, stage + (b ^ 1) * kStageWords, lane);
+        const ChunkMeta after = header(k + 2 * nw);
+        cp_async_wait<1>();
+        __syncwarp();
+        fn(k, cur, stage + b * kStageWords);
+        __syncwarp();
+        cur = next;
+        next = after;
+        b ^= 1;
+    }
+    cp_async_wait<0>();
 }
 
 // A warp's output space: it takes `slab` bytes of the arena at a time (its
@@ -1947,26 +1993,30 @@ __global__ void sum_mask_bytes_kernel(const uint8_t *mask, const unsigned long l
 }
 
 // ------------------------------------------------------------ readout / norm
-template <typename R>
+// One warp per chunk, straight from the packed words to the output: bound by
+// the complex128 amplitudes it writes.
+template <typename R, int kPL>
 __global__ void readout_kernel(const ChunkMeta *meta, const uint32_t *arena, const uint8_t *mask, int B, int C,
                                CodecParams p, uint64_t chunk0, uint64_t nchunks, double *out, double scale) {
-    __shared__ __align__(16) uint32_t stage[kPassThreads / 32][kStageWords];
-    __shared__ R vals[kPassThreads / 32][2 << kMaxChunkLog2];
+    using T = typename Cplx<R>::T;
+    __shared__ __align__(16) uint32_t stage[kPassThreads / 32][2 * kStageWords];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ncomp = 2 << C, per_lane = ncomp >> 5;
-    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t k = gw; k < nchunks; k += nw) {
-        const uint64_t chunk = chunk0 + k;
-        double *o = out + k * (uint64_t)ncomp;
-        if (!mask[chunk >> (B - C)]) {
-            for (int i = 0; i < per_lane; ++i) o[lane + 32 * i] = 0.0;
-            continue;
-        }
-        decode_chunk<R>(arena, meta[chunk], per_lane, p, vals[warp], stage[warp], lane);
-        for (int i = 0; i < per_lane; ++i) o[lane + 32 * i] = (double)vals[warp][lane + 32 * i] * scale;
-        __syncwarp();
-    }
+    const int per_lane = (2 << C) >> 5;
+    const PairLanes<kPL> pl(per_lane, lane);
+    const bool wide = (reinterpret_cast<size_t>(out) & 15) == 0;
+    stream_chunks(meta, arena, mask, B, C, chunk0, nchunks, stage[warp], lane,
+                  [&](uint64_t k, const ChunkMeta md, const uint32_t *src) {
+                      double *const o = out + ((k << C) + 16 * pl.i0 + pl.k) * 2;
+                      decode_pairs<R, false, kPL, false>(md, per_lane, p, src, lane, [&](int i, T v) {
+                          const double2 d = make_double2((double)v.x * scale, (double)v.y * scale);
+                          if (wide) {
+                              __stcs(reinterpret_cast<double2 *>(o + 32 * i), d);
+                          } else {
+                              o[32 * i] = d.x;
+                              o[32 * i + 1] = d.y;
+                          }
+                      });
+                  });
 }
 
 // ------------------------------------------------------------ sampling
@@ -2070,25 +2120,22 @@ __global__ void sample_in_block_kernel(const ChunkMeta *meta, const uint32_t *ar
     }
 }
 
-template <typename R>
+template <typename R, int kPL>
 __global__ void norm_kernel(const ChunkMeta *meta, const uint32_t *arena, const uint8_t *mask, int B, int C,
                             CodecParams p, uint64_t nchunks, double *out) {
-    __shared__ __align__(16) uint32_t stage[kPassThreads / 32][kStageWords];
-    __shared__ R vals[kPassThreads / 32][2 << kMaxChunkLog2];
+    using T = typename Cplx<R>::T;
+    __shared__ __align__(16) uint32_t stage[kPassThreads / 32][2 * kStageWords];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ncomp = 2 << C, per_lane = ncomp >> 5;
-    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    double acc = 0.0;
-    for (uint64_t chunk = gw; chunk < nchunks; chunk += nw) {
-        if (!mask[chunk >> (B - C)]) continue;
-        decode_chunk<R>(arena, meta[chunk], per_lane, p, vals[warp], stage[warp], lane);
-        for (int i = 0; i < per_lane; ++i) {
-            const double v = (double)vals[warp][lane + 32 * i];
-            acc = fma(v, v, acc);
-        }
-        __syncwarp();
-    }
+    const int per_lane = (2 << C) >> 5;
+    double re = 0.0, im = 0.0;
+    stream_chunks(meta, arena, mask, B, C, 0, nchunks, stage[warp], lane,
+                  [&](uint64_t, const ChunkMeta md, const uint32_t *src) {
+                      decode_pairs<R, false, kPL, false>(md, per_lane, p, src, lane, [&](int, T v) {
+                          re = fma((double)v.x, (double)v.x, re);
+                          im = fma((double)v.y, (double)v.y, im);
+                      });
+                  });
+    double acc = re + im;
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0 && acc != 0.0) atomicAdd(out, acc);
 }
@@ -3166,8 +3213,9 @@ cudaError_t launch_readout(bool f64, const ChunkMeta *meta, const uint32_t *aren
                            CodecParams p, uint64_t chunk0, uint64_t nchunks, double *out, double scale,
                            cudaStream_t s) {
     const unsigned grid = grid_for(nchunks, kPassThreads / 32, 8);
-    if (f64) readout_kernel<double><<<grid, kPassThreads, 0, s>>>(meta, arena, mask, B, C, p, chunk0, nchunks, out, scale);
-    else readout_kernel<float><<<grid, kPassThreads, 0, s>>>(meta, arena, mask, B, C, p, chunk0, nchunks, out, scale);
+    auto run = [&](auto kern) { kern<<<grid, kPassThreads, 0, s>>>(meta, arena, mask, B, C, p, chunk0, nchunks, out, scale); };
+    if (C == kMaxChunkLog2) f64 ? run(readout_kernel<double, kMaxPerLane>) : run(readout_kernel<float, kMaxPerLane>);
+    else f64 ? run(readout_kernel<double, 0>) : run(readout_kernel<float, 0>);
     return cudaGetLastError();
 }
 
@@ -3202,8 +3250,9 @@ cudaError_t launch_sample_in_block(bool f64, const ChunkMeta *meta, const uint32
 cudaError_t launch_norm(bool f64, const ChunkMeta *meta, const uint32_t *arena, const uint8_t *mask, int B, int C,
                         CodecParams p, uint64_t nchunks, double *out, cudaStream_t s) {
     const unsigned grid = grid_for(nchunks, kPassThreads / 32, 8);
-    if (f64) norm_kernel<double><<<grid, kPassThreads, 0, s>>>(meta, arena, mask, B, C, p, nchunks, out);
-    else norm_kernel<float><<<grid, kPassThreads, 0, s>>>(meta, arena, mask, B, C, p, nchunks, out);
+    auto run = [&](auto kern) { kern<<<grid, kPassThreads, 0, s>>>(meta, arena, mask, B, C, p, nchunks, out); };
+    if (C == kMaxChunkLog2) f64 ? run(norm_kernel<double, kMaxPerLane>) : run(norm_kernel<float, kMaxPerLane>);
+    else f64 ? run(norm_kernel<double, 0>) : run(norm_kernel<float, 0>);
     return cudaGetLastError();
 }
 
