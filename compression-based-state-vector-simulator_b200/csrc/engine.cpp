@@ -756,23 +756,33 @@ bool program_op(int code, uint32_t *what) {
 // The program of one pass (internal.h): its sweeps (op ranges relative to
 // ops), ops and fixed matrices in the state's precision.  False when the pass
 // is too long for one.
-bool build_program(const std::vector<qs::Sweep> &sweeps, const qs::ROp *ops, const std::vector<cplx> &pool, bool f64,
-                   qs::PassProgram *out) {
+bool build_program(const qs::Sweep *sweeps, size_t nsweeps, int RB, const qs::ROp *ops, const std::vector<cplx> &pool,
+                   bool f64, qs::PassProgram *out) {
     std::memset(out, 0, sizeof(*out));
-    if (sweeps.size() > (size_t)qs::kProgSweeps) return false;
+    if (nsweeps > (size_t)qs::kProgSweeps) return false;
     const size_t entry = f64 ? 16 : 8;
     size_t used = 0;
-    out->nsweeps = (int32_t)sweeps.size();
-    for (size_t w = 0; w < sweeps.size(); ++w) {
+    out->nsweeps = (int32_t)nsweeps;
+    for (size_t w = 0; w < nsweeps; ++w) {
         const qs::Sweep &sw = sweeps[w];
         qs::ProgSweep &ps = out->sweeps[w];
         if (sw.g1 > qs::kProgOps) return false;
         ps.g0 = sw.g0;
         ps.g1 = sw.g1;
-        for (int k = 0; k < qs::kRegBits; ++k) ps.sbits[k] = sw.sbits[k];
+        for (int k = 0; k < RB; ++k) ps.sbits[k] = sw.sbits[k];
         for (int k = sw.g0; k < sw.g1; ++k) {
             const qs::ROp &o = ops[k];
             qs::ProgOp &p = out->ops[k];
+            if (o.code == qs::OPC_SUM) {
+                p.what = qs::kProgSum;
+                p.mat = o.vstride;
+                p.stride = o.pad;
+                if (o.sel[0] & qs::kSelRuns)
+                    p.s1 = (((1u << o.sel[1]) - 1u) << (o.sel[0] & 31u)) | (((1u << o.sel[3]) - 1u) << o.sel[2]);
+                else
+                    for (int j = 0; j < o.nsel; ++j) p.s1 |= 1u << o.sel[j];
+                continue;
+            }
             if (!program_op(o.code, &p.what)) return false;
             p.stride = o.vstride;
             if (o.code == qs::OPC_SCALAR) ps.scalar = 1;
@@ -1607,7 +1617,7 @@ static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGat
         }
         dp.nsweeps = (uint32_t)swp.size();
         auto prog = std::make_shared<qs::PassProgram>();
-        if (build_program(swp, ops.data() + op0, pool, h->f64, prog.get())) dp.prog = prog;
+        if (build_program(swp.data(), swp.size(), RB, ops.data() + op0, pool, h->f64, prog.get())) dp.prog = prog;
         sw.insert(sw.end(), swp.begin(), swp.end());
         out->push_back(dp);
     }
@@ -3813,7 +3823,8 @@ qs_status qs_dense_apply_gates(qs_dense *h, const qs_gate *gates, size_t count) 
             return dfail(h, QS_ERR_ARG, "a pass needs more outer selector qubits than the planner allows");
         fuse_half_chains(&ops, op0, swp);
         progs.emplace_back();
-        if (!build_program(swp, ops.data() + op0, pool, h->f64, &progs.back())) progs.back().nsweeps = -1;
+        if (!build_program(swp.data(), swp.size(), RB, ops.data() + op0, pool, h->f64, &progs.back()))
+            progs.back().nsweeps = -1;
         outers.push_back(outer);
         op_offsets.push_back(op0);
         sweep_ranges.push_back({sw.size(), swp.size()});
@@ -4103,8 +4114,8 @@ qs_status qs_dense_adjoint(qs_dense *psi, qs_dense *lam, const qs_gate *gates, c
     std::vector<uint32_t> ids(count);
     for (size_t i = 0; i < count; ++i) ids[i] = (uint32_t)i;
     // commuting gates may change places (the argument at qs_adjoint holds here)
-    auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, cg, C, jmax, std::min(jmax, 3), C, n)
-                                             : plan_passes(ids, cg, C, jmax, std::min(jmax, 3), C, n);
+    auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, cg, C, jmax, jmax, C, n)
+                                             : plan_passes(ids, cg, C, jmax, jmax, C, n);
     // every launch's gate records (at most 128 parametric gates each) are
     // built first and uploaded at once; the launches then run back to back
     // and their slot sums are read back with one copy at the end
@@ -4176,6 +4187,12 @@ qs_status qs_dense_adjoint(qs_dense *psi, qs_dense *lam, const qs_gate *gates, c
         for (Launch &L : launches)
             L.fused = plan_dual_sweeps(cg, L.gates, slots, gen_x, gen_z, L.tile, C, RB, &all_sw, &all_rops, &all_pool,
                                        &L.sweeps);
+    std::vector<qs::PassProgram> progs(launches.size());
+    std::vector<char> has_prog(launches.size(), 0);
+    for (size_t l = 0; l < launches.size(); ++l)
+        if (launches[l].fused)
+            has_prog[l] = build_program(all_sw.data() + launches[l].sweeps.sw_off, launches[l].sweeps.nsw, RB,
+                                        all_rops.data() + launches[l].sweeps.rop_off, all_pool, psi->f64, &progs[l]);
     std::vector<double> acc(2 * (size_t)nslots, 0.0);
     double *dout = nullptr;
     qs::AdjGate *dg = nullptr;
@@ -4204,7 +4221,8 @@ qs_status qs_dense_adjoint(qs_dense *psi, qs_dense *lam, const qs_gate *gates, c
         e = cudaMemcpyAsync(dpool, psi->f64 ? (const void *)pool_d.data() : (const void *)pool_f.data(), pool_bytes,
                             cudaMemcpyHostToDevice, psi->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(dout, 0, std::max<size_t>(1, 2 * nout) * sizeof(double), psi->stream);
-    for (const Launch &L : launches) {
+    for (size_t l = 0; l < launches.size(); ++l) {
+        const Launch &L = launches[l];
         if (e != cudaSuccess) break;
         qs::AdjPassArgs a{};
         if (L.fused) {
@@ -4227,7 +4245,7 @@ qs_status qs_dense_adjoint(qs_dense *psi, qs_dense *lam, const qs_gate *gates, c
         a.lam = lam->state;
         a.out = dout + 2 * L.out_off;
         a.nslots = (int)L.local_to_global.size();
-        e = qs::launch_adjoint_pass(psi->f64, a, psi->stream);
+        e = qs::launch_adjoint_pass(psi->f64, a, has_prog[l] ? &progs[l] : nullptr, psi->stream);
     }
     std::vector<double> h(2 * nout);
     if (e == cudaSuccess && nout)

@@ -129,15 +129,18 @@ static_assert(sizeof(KGate) == 288, "KGate layout");
 //             variant * stride), else its entries lie in mats at entry `mat`
 //   variant   ((W >> s1) & m1) + (((W >> s2) & m2) << l1); with kProgSelList
 //             s1 and m1 hold the selector positions as bytes instead
+//   kProgSum  (two-state passes) OPC_SUM: mat = slot, stride = xs << 4 | zs, the
+//             sign is the parity of W & s1
 // One-hot bits instead of a code: the device tests them one after another, and
 // each test joins two paths only.  A switch over all bodies joined some forty,
 // and the compiler then copied the whole register group (64 registers in
 // double precision) after every op.
 constexpr uint32_t kProgScalar = 1, kProgAcc = 2, kProgHalf = 4, kProgHalfPending = 8, kProgDiag = 16, kProgM2 = 32,
-                   kProgX = 64, kProgHalf4 = 128, kProgDiag4 = 256, kProgM4 = 512, kProgSwap = 1024;
+                   kProgX = 64, kProgHalf4 = 128, kProgDiag4 = 256, kProgM4 = 512, kProgSwap = 1024,
+                   kProgSum = 2048;
 constexpr uint32_t kProgVar = 1u << 14, kProgSelList = 1u << 15;
 constexpr int kProgWhere = 16;
-constexpr int kProgOps = 80, kProgSweeps = 16, kProgMatBytes = 6144;
+constexpr int kProgOps = 192, kProgSweeps = 32, kProgMatBytes = 8192;
 struct ProgOp {
     uint32_t what, mat, stride, s1, m1, s2, m2, l1;
 };
@@ -399,7 +402,8 @@ struct DualPassArgs {
 
 // ---- launchers (kernels.cu); all asynchronous on `stream` ----
 cudaError_t launch_dual_pass(bool f64, const DualPassArgs &a, cudaStream_t stream);
-cudaError_t launch_adjoint_pass(bool f64, const AdjPassArgs &a, cudaStream_t stream);
+// prog: the pass's program (its sweeps hold a.rb register bits) or NULL.
+cudaError_t launch_adjoint_pass(bool f64, const AdjPassArgs &a, const PassProgram *prog, cudaStream_t stream);
 cudaError_t launch_dense_transition(bool f64, const void *bra, const void *ket, int n, const PauliTerm *terms,
                                     int nterms, double *out, cudaStream_t stream);
 // out = sum_t coef_t P_t in (coefs complex interleaved; PauliTerm global masks, ny folded into coefs)

@@ -345,15 +345,30 @@ __device__ __forceinline__ void tile_sweeps_body(typename Cplx<R>::T *tile, int 
     }
 }
 // One op of a program.  Its class and place are uniform, so each branch is.
-template <int RB, typename T>
-__device__ __forceinline__ void apply_prog_op(T (&v)[1 << RB], T &z, T &zh, const PassProgram &pr, int k,
-                                              const T *__restrict__ pool, uint32_t W) {
+// kTwo: the same op on a second group w (the two states of a backward pass,
+// whose pending factors z and zh are the same).
+template <int RB, bool kTwo, typename T>
+__device__ __forceinline__ void apply_prog_op(T (&v)[1 << RB], T (&w)[kTwo ? 1 << RB : 1], T &z, T &zh,
+                                              const PassProgram &pr, int k, const T *__restrict__ pool, uint32_t W) {
     constexpr int NS = 1 << RB;
-    static_assert(RB == 4, "the place bits of ProgOp name four register bits");
     const ProgOp &o = pr.ops[k];
     const T *const mats = reinterpret_cast<const T *>(pr.mats);
     const uint32_t what = o.what;
     const uint32_t at = what >> kProgWhere;
+#define QS_ON1(F, A, ...)                                           \
+    do {                                                            \
+        if constexpr ((A) < RB) {                                   \
+            F<NS, (A)>(v __VA_OPT__(, ) __VA_ARGS__);               \
+            if constexpr (kTwo) F<NS, (A)>(w __VA_OPT__(, ) __VA_ARGS__); \
+        }                                                           \
+    } while (0)
+#define QS_ON2(F, A, B, ...)                                        \
+    do {                                                            \
+        if constexpr ((B) < RB) {                                   \
+            F<NS, (A), (B)>(v __VA_OPT__(, ) __VA_ARGS__);          \
+            if constexpr (kTwo) F<NS, (A), (B)>(w __VA_OPT__(, ) __VA_ARGS__); \
+        }                                                           \
+    } while (0)
     T e0, e1, e2, e3;
     if (what & kProgVar) {
         uint32_t var;
@@ -387,66 +402,68 @@ __device__ __forceinline__ void apply_prog_op(T (&v)[1 << RB], T &z, T &zh, cons
             e0 = cmul(zh, e0);
             zh = c_one<T>();
         }
-        if (at & 1) r_half2<NS, 0>(v, e0);
-        if (at & 2) r_half2<NS, 1>(v, e0);
-        if (at & 4) r_half2<NS, 2>(v, e0);
-        if (at & 8) r_half2<NS, 3>(v, e0);
+        if (at & 1) QS_ON1(r_half2, 0, e0);
+        if (at & 2) QS_ON1(r_half2, 1, e0);
+        if (at & 4) QS_ON1(r_half2, 2, e0);
+        if (at & 8) QS_ON1(r_half2, 3, e0);
         return;
     }
     if (what & kProgM4) {
-        if (at & 1) r_4x4<NS, 0, 1>(v, mats + o.mat);
-        if (at & 2) r_4x4<NS, 0, 2>(v, mats + o.mat);
-        if (at & 4) r_4x4<NS, 0, 3>(v, mats + o.mat);
-        if (at & 8) r_4x4<NS, 1, 2>(v, mats + o.mat);
-        if (at & 16) r_4x4<NS, 1, 3>(v, mats + o.mat);
-        if (at & 32) r_4x4<NS, 2, 3>(v, mats + o.mat);
+        if (at & 1) QS_ON2(r_4x4, 0, 1, mats + o.mat);
+        if (at & 2) QS_ON2(r_4x4, 0, 2, mats + o.mat);
+        if (at & 4) QS_ON2(r_4x4, 0, 3, mats + o.mat);
+        if (at & 8) QS_ON2(r_4x4, 1, 2, mats + o.mat);
+        if (at & 16) QS_ON2(r_4x4, 1, 3, mats + o.mat);
+        if (at & 32) QS_ON2(r_4x4, 2, 3, mats + o.mat);
         return;
     }
     if (what & kProgM2) {
-        if (at & 1) r_2x2<NS, 0>(v, e0, e1, e2, e3);
-        if (at & 2) r_2x2<NS, 1>(v, e0, e1, e2, e3);
-        if (at & 4) r_2x2<NS, 2>(v, e0, e1, e2, e3);
-        if (at & 8) r_2x2<NS, 3>(v, e0, e1, e2, e3);
+        if (at & 1) QS_ON1(r_2x2, 0, e0, e1, e2, e3);
+        if (at & 2) QS_ON1(r_2x2, 1, e0, e1, e2, e3);
+        if (at & 4) QS_ON1(r_2x2, 2, e0, e1, e2, e3);
+        if (at & 8) QS_ON1(r_2x2, 3, e0, e1, e2, e3);
         return;
     }
     if (what & kProgHalf4) {
-        if (at & 1) r_half4<NS, 0, 1>(v, e0, e1, e2);
-        if (at & 2) r_half4<NS, 0, 2>(v, e0, e1, e2);
-        if (at & 4) r_half4<NS, 0, 3>(v, e0, e1, e2);
-        if (at & 8) r_half4<NS, 1, 2>(v, e0, e1, e2);
-        if (at & 16) r_half4<NS, 1, 3>(v, e0, e1, e2);
-        if (at & 32) r_half4<NS, 2, 3>(v, e0, e1, e2);
+        if (at & 1) QS_ON2(r_half4, 0, 1, e0, e1, e2);
+        if (at & 2) QS_ON2(r_half4, 0, 2, e0, e1, e2);
+        if (at & 4) QS_ON2(r_half4, 0, 3, e0, e1, e2);
+        if (at & 8) QS_ON2(r_half4, 1, 2, e0, e1, e2);
+        if (at & 16) QS_ON2(r_half4, 1, 3, e0, e1, e2);
+        if (at & 32) QS_ON2(r_half4, 2, 3, e0, e1, e2);
         return;
     }
     if (what & kProgDiag) {
-        if (at & 1) r_diag2<NS, 0>(v, e0, e1);
-        if (at & 2) r_diag2<NS, 1>(v, e0, e1);
-        if (at & 4) r_diag2<NS, 2>(v, e0, e1);
-        if (at & 8) r_diag2<NS, 3>(v, e0, e1);
+        if (at & 1) QS_ON1(r_diag2, 0, e0, e1);
+        if (at & 2) QS_ON1(r_diag2, 1, e0, e1);
+        if (at & 4) QS_ON1(r_diag2, 2, e0, e1);
+        if (at & 8) QS_ON1(r_diag2, 3, e0, e1);
         return;
     }
     if (what & kProgDiag4) {
-        if (at & 1) r_diag4<NS, 0, 1>(v, e0, e1, e2, e3);
-        if (at & 2) r_diag4<NS, 0, 2>(v, e0, e1, e2, e3);
-        if (at & 4) r_diag4<NS, 0, 3>(v, e0, e1, e2, e3);
-        if (at & 8) r_diag4<NS, 1, 2>(v, e0, e1, e2, e3);
-        if (at & 16) r_diag4<NS, 1, 3>(v, e0, e1, e2, e3);
-        if (at & 32) r_diag4<NS, 2, 3>(v, e0, e1, e2, e3);
+        if (at & 1) QS_ON2(r_diag4, 0, 1, e0, e1, e2, e3);
+        if (at & 2) QS_ON2(r_diag4, 0, 2, e0, e1, e2, e3);
+        if (at & 4) QS_ON2(r_diag4, 0, 3, e0, e1, e2, e3);
+        if (at & 8) QS_ON2(r_diag4, 1, 2, e0, e1, e2, e3);
+        if (at & 16) QS_ON2(r_diag4, 1, 3, e0, e1, e2, e3);
+        if (at & 32) QS_ON2(r_diag4, 2, 3, e0, e1, e2, e3);
         return;
     }
     if (what & kProgX) {
-        if (at & 1) r_x<NS, 0>(v);
-        if (at & 2) r_x<NS, 1>(v);
-        if (at & 4) r_x<NS, 2>(v);
-        if (at & 8) r_x<NS, 3>(v);
+        if (at & 1) QS_ON1(r_x, 0);
+        if (at & 2) QS_ON1(r_x, 1);
+        if (at & 4) QS_ON1(r_x, 2);
+        if (at & 8) QS_ON1(r_x, 3);
     } else {  // kProgSwap
-        if (at & 1) r_swap<NS, 0, 1>(v);
-        if (at & 2) r_swap<NS, 0, 2>(v);
-        if (at & 4) r_swap<NS, 0, 3>(v);
-        if (at & 8) r_swap<NS, 1, 2>(v);
-        if (at & 16) r_swap<NS, 1, 3>(v);
-        if (at & 32) r_swap<NS, 2, 3>(v);
+        if (at & 1) QS_ON2(r_swap, 0, 1);
+        if (at & 2) QS_ON2(r_swap, 0, 2);
+        if (at & 4) QS_ON2(r_swap, 0, 3);
+        if (at & 8) QS_ON2(r_swap, 1, 2);
+        if (at & 16) QS_ON2(r_swap, 1, 3);
+        if (at & 32) QS_ON2(r_swap, 2, 3);
     }
+#undef QS_ON1
+#undef QS_ON2
 }
 
 // The sweeps of a pass whose program is a kernel parameter.
@@ -480,7 +497,8 @@ __device__ __forceinline__ void tile_sweeps_prog(typename Cplx<R>::T *tile, int 
 #pragma unroll
             for (int s = 0; s < NS; ++s) v[s] = g[olo[s & 3] + ohi[s >> 2]];
             T z = c_one<T>(), zh = c_one<T>();
-            for (int k = sw.g0; k < sw.g1; ++k) apply_prog_op<RB>(v, z, zh, pr, k, pool, W);
+            T none[1];
+            for (int k = sw.g0; k < sw.g1; ++k) apply_prog_op<RB, false>(v, none, z, zh, pr, k, pool, W);
             if (sw.scalar) {
 #pragma unroll
                 for (int s = 0; s < NS; ++s) v[s] = cmul(z, v[s]);
@@ -2714,6 +2732,130 @@ __device__ void dual_tile_sweeps(typename Cplx<R>::T *tA, typename Cplx<R>::T *t
     }
 }
 
+// The backward pass with its ops as a program (default geometry).  Each thread
+// holds the groups of psi and lambda at the same 2^RB tile positions.  Both
+// tiles load asynchronously, the CTA's next tiles are prefetched into L2.
+template <typename R, int RB, int kC, int kJ>
+__global__ void __launch_bounds__(kAdjThreads, 2)
+    adjoint_prog_kernel(const __grid_constant__ AdjPassArgs a, const __grid_constant__ PassProgram pr) {
+    using T = typename Cplx<R>::T;
+    constexpr int NS = 1 << RB, nb = kC + kJ, size = 1 << nb, cmask = (1 << kC) - 1, groups = 1 << (nb - RB);
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double s_acc[2 * kMaxAdjSlots];
+    __shared__ uint64_t s_off[1 << kJ];
+    __shared__ int32_t s_tq[kMaxTileQubits];
+    __shared__ int8_t s_oq[kMaxOuterSel];
+    const int lane = threadIdx.x & 31;
+    T *const tp = reinterpret_cast<T *>(smem);
+    T *const tl = reinterpret_cast<T *>(smem + tile_bytes<R>(nb));
+    T *const psi = reinterpret_cast<T *>(a.psi);
+    T *const lam = reinterpret_cast<T *>(a.lam);
+    const T *const pool = reinterpret_cast<const T *>(a.pool);
+    for (int i = threadIdx.x; i < 2 * a.nslots; i += blockDim.x) s_acc[i] = 0.0;
+    if (threadIdx.x < kMaxTileQubits) s_tq[threadIdx.x] = a.tq[threadIdx.x];
+    if (threadIdx.x < kMaxOuterSel) s_oq[threadIdx.x] = a.outer_q[threadIdx.x];
+    __syncthreads();
+    for (int c = threadIdx.x; c < (1 << kJ); c += blockDim.x) s_off[c] = deposit_bits((uint32_t)c, s_tq, kJ) << kC;
+    __syncthreads();
+    for (uint64_t tile_id = blockIdx.x; tile_id < a.n_tiles; tile_id += gridDim.x) {
+        const uint64_t base_amp = insert_zero_bits(tile_id, s_tq, kJ) << kC;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < size; e += kAdjThreads) {
+            const uint64_t amp = base_amp + s_off[e >> kC] + (e & cmask);
+            cp_async_elem<sizeof(T)>(&tp[pos<R>(e)], &psi[amp]);
+            cp_async_elem<sizeof(T)>(&tl[pos<R>(e)], &lam[amp]);
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+        if (tile_id + gridDim.x < a.n_tiles) {
+            const uint64_t nx = insert_zero_bits(tile_id + gridDim.x, s_tq, kJ) << kC;
+            constexpr int kLine = 128 / sizeof(T);
+            for (int e = threadIdx.x * kLine; e < size; e += kAdjThreads * kLine) {
+                const uint64_t amp = nx + s_off[e >> kC] + (e & cmask);
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(psi + amp));
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(lam + amp));
+            }
+        }
+        const uint32_t wo = outer_word(base_amp, s_oq, a.nouter) << nb;
+        for (int sidx = 0; sidx < pr.nsweeps; ++sidx) {
+            const ProgSweep &sw = pr.sweeps[sidx];
+            int po[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                po[s] = 0;
+#pragma unroll
+                for (int k = 0; k < RB; ++k)
+                    if ((s >> k) & 1) po[s] += pos<R>(1 << sw.sbits[k]);
+            }
+            // every thread runs the same number of groups (groups is a multiple
+            // of the CTA size or smaller than it): the warp sums see 32 lanes
+            for (int g0 = 0; g0 < groups; g0 += kAdjThreads) {
+                const int grp = g0 + threadIdx.x;
+                const bool live = grp < groups;
+                int base = live ? grp : 0;
+#pragma unroll
+                for (int k = 0; k < RB; ++k) {
+                    const int t = sw.sbits[k];
+                    base = ((base >> t) << (t + 1)) | (base & ((1 << t) - 1));
+                }
+                const uint32_t W = (uint32_t)base | wo;
+                T *const gp = tp + pos<R>(base), *const gl = tl + pos<R>(base);
+                T v[NS], w[NS];
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    v[s] = gp[po[s]];
+                    w[s] = gl[po[s]];
+                }
+                T z = c_one<T>(), zh = c_one<T>();
+                for (int k = sw.g0; k < sw.g1; ++k) {
+                    if (pr.ops[k].what & kProgSum) {
+                        const ProgOp &o = pr.ops[k];
+                        double re = 0.0, im = 0.0;
+                        group_pauli_sum_any<RB>(v, w, (int)(o.stride >> 4), (int)(o.stride & 15u), re, im);
+                        // the groups' pending factor enters as |z|^2
+                        double f = (double)z.x * (double)z.x + (double)z.y * (double)z.y;
+                        if (__popc(W & o.s1) & 1) f = -f;
+                        if (!live) f = 0.0;
+                        // warp sums of both parts: the first exchange leaves each
+                        // half-warp with one of them
+                        const double mine = lane < 16 ? re : im, other = lane < 16 ? im : re;
+                        double acc = f * mine + __shfl_xor_sync(0xffffffffu, f * other, 16);
+#pragma unroll
+                        for (int d = 8; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+                        if ((lane & 15) == 0) atomicAdd(&s_acc[2 * o.mat + (lane >> 4)], acc);
+                    } else {
+                        apply_prog_op<RB, true>(v, w, z, zh, pr, k, pool, W);
+                    }
+                }
+                if (sw.scalar) {
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) {
+                        v[s] = cmul(z, v[s]);
+                        w[s] = cmul(z, w[s]);
+                    }
+                }
+                if (live) {
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) {
+                        gp[po[s]] = v[s];
+                        gl[po[s]] = w[s];
+                    }
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll 4
+        for (int e = threadIdx.x; e < size; e += kAdjThreads) {
+            const uint64_t amp = base_amp + s_off[e >> kC] + (e & cmask);
+            psi[amp] = tp[pos<R>(e)];
+            lam[amp] = tl[pos<R>(e)];
+        }
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < 2 * a.nslots; i += blockDim.x)
+        if (s_acc[i] != 0.0) atomicAdd(&a.out[i], s_acc[i]);
+}
+
 // kC, kJ: chunk log2 and tile qubits above the chunk as compile-time
 // constants (0: read from the args), as for pass_kernel.
 template <typename R, int kC, int kJ>
@@ -3394,20 +3536,33 @@ static cudaError_t launch_adjoint_pass_kc(const AdjPassArgs &a, cudaStream_t s) 
 }
 
 // The uncompressed adjoint's default geometry: 2^5-amplitude chunks and
-// tiles of 2^11 (complex128) or 2^12 (complex64) amplitudes.
+// tiles of 2^11 (complex128) or 2^12 (complex64) amplitudes, with a program.
 template <typename R>
-static cudaError_t launch_adjoint_pass_t(const AdjPassArgs &a, cudaStream_t s) {
+static cudaError_t launch_adjoint_pass_t(const AdjPassArgs &a, const PassProgram *prog, cudaStream_t s) {
     if (a.nslots > kMaxAdjSlots) return cudaErrorInvalidValue;
-    if (a.nsweeps > 0 && (a.rb != (sizeof(R) == 8 ? kDualRegBitsF64 : kDualRegBitsF32) || a.C + a.j < a.rb ||
-                          a.nouter < 0 || a.nouter > kMaxOuterSel || !a.sweeps || !a.rops || !a.pool))
+    constexpr int kRB = sizeof(R) == 8 ? kDualRegBitsF64 : kDualRegBitsF32;
+    if (a.nsweeps > 0 && (a.rb != kRB || a.C + a.j < a.rb || a.nouter < 0 || a.nouter > kMaxOuterSel || !a.sweeps ||
+                          !a.rops || !a.pool))
         return cudaErrorInvalidValue;
     constexpr int kAC = 5, kAJ = sizeof(R) == 8 ? 6 : 7;
-    if (a.C == kAC && a.j == kAJ) return launch_adjoint_pass_kc<R, kAC, kAJ>(a, s);
-    return launch_adjoint_pass_kc<R, 0, 0>(a, s);
+    if (a.C != kAC || a.j != kAJ || !prog || a.nsweeps == 0) return launch_adjoint_pass_kc<R, 0, 0>(a, s);
+    const size_t smem = 2 * tile_bytes<R>(kAC + kAJ);
+    auto kern = adjoint_prog_kernel<R, kRB, kAC, kAJ>;
+    cudaError_t e = ensure_dyn_smem(kern, smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kAdjThreads, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    uint64_t grid = (uint64_t)per_sm * sm_count();
+    if (grid > a.n_tiles) grid = a.n_tiles;
+    if (grid == 0) grid = 1;
+    kern<<<(unsigned)grid, kAdjThreads, smem, s>>>(a, *prog);
+    return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_pass(bool f64, const AdjPassArgs &a, cudaStream_t s) {
-    return f64 ? launch_adjoint_pass_t<double>(a, s) : launch_adjoint_pass_t<float>(a, s);
+cudaError_t launch_adjoint_pass(bool f64, const AdjPassArgs &a, const PassProgram *prog, cudaStream_t s) {
+    return f64 ? launch_adjoint_pass_t<double>(a, prog, s) : launch_adjoint_pass_t<float>(a, prog, s);
 }
 
 // Host code may not use g_noalloc_words directly: in host code the name is a
