@@ -344,6 +344,77 @@ std::vector<qs::Sweep> plan_sweeps(const std::vector<qs::KGate> &kg, size_t g0, 
     return out;
 }
 
+// An order of the gates [g0, end) in which plan_sweeps makes fewer sweeps, as
+// indices into kg: a sweep takes, lowest index first and repeatedly, every
+// gate whose earlier gates it does not commute with are done and whose mixing
+// bits still fit RB register bits (the rule of plan_passes_dag, within a
+// pass).  Each sweep costs every amplitude a trip through shared memory.
+std::vector<size_t> sweep_order(const std::vector<qs::KGate> &kg, size_t g0, int RB) {
+    const size_t G = kg.size() - g0;
+    std::vector<std::vector<uint32_t>> succ(G);
+    std::vector<int> indeg(G, 0);
+    {
+        std::vector<int> last_mix(64, -1);
+        std::vector<std::vector<uint32_t>> users(64);
+        std::vector<uint32_t> preds;
+        for (size_t i = 0; i < G; ++i) {
+            const qs::KGate &g = kg[g0 + i];
+            preds.clear();
+            for (int b = 0; b < g.nq; ++b) {
+                const int q = g.q[b];
+                if (last_mix[q] >= 0) preds.push_back((uint32_t)last_mix[q]);
+                if ((g.mixmask >> b) & 1) {
+                    preds.insert(preds.end(), users[q].begin(), users[q].end());
+                    last_mix[q] = (int)i;
+                    users[q].clear();
+                } else {
+                    users[q].push_back((uint32_t)i);
+                }
+            }
+            std::sort(preds.begin(), preds.end());
+            preds.erase(std::unique(preds.begin(), preds.end()), preds.end());
+            for (uint32_t p : preds) {
+                succ[p].push_back((uint32_t)i);
+                ++indeg[i];
+            }
+        }
+    }
+    std::vector<uint32_t> need(G, 0);
+    for (size_t i = 0; i < G; ++i)
+        for (int b = 0; b < kg[g0 + i].nq; ++b)
+            if ((kg[g0 + i].mixmask >> b) & 1) need[i] |= 1u << kg[g0 + i].tpos[b];
+    std::vector<size_t> order;
+    order.reserve(G);
+    std::set<uint32_t> ready;
+    for (size_t i = 0; i < G; ++i)
+        if (indeg[i] == 0) ready.insert((uint32_t)i);
+    uint32_t cur = 0;
+    while (!ready.empty()) {
+        auto it = ready.begin();
+        while (it != ready.end() && __builtin_popcount(cur | need[*it]) > RB) ++it;
+        if (it == ready.end()) {
+            cur = 0;  // the sweep is full
+            it = ready.begin();
+        }
+        const uint32_t i = *it;
+        ready.erase(it);
+        cur |= need[i];
+        order.push_back(g0 + i);
+        for (uint32_t sx : succ[i])
+            if (--indeg[sx] == 0) ready.insert(sx);
+    }
+    return order;
+}
+
+// kg[g0, end) put into sweep_order.
+void order_for_sweeps(std::vector<qs::KGate> *kg, size_t g0, int RB) {
+    const std::vector<size_t> order = sweep_order(*kg, g0, RB);
+    std::vector<qs::KGate> out;
+    out.reserve(order.size());
+    for (size_t i : order) out.push_back((*kg)[i]);
+    std::copy(out.begin(), out.end(), kg->begin() + g0);
+}
+
 // Resolve the gates [g0, g1) of a pass against their sweeps into op records
 // and sub-matrix variants (appended to *ops and *pool).  Sweep gate ranges are
 // relative to g0; op k of the pass is gate g0 + k.
@@ -1032,6 +1103,19 @@ bool plan_dual_sweeps(const std::vector<CGate> &cg, const std::vector<uint32_t> 
         sum_slot.push_back(-1);
         gid.push_back(gi);
     }
+    {
+        // a sum keeps its place before every gate that does not commute with
+        // its generator: it carries its gate's qubits and mixing bits
+        const std::vector<size_t> order = sweep_order(kg, 0, RB);
+        const auto kg0 = kg;
+        const auto sum0 = sum_slot;
+        const auto gid0 = gid;
+        for (size_t i = 0; i < order.size(); ++i) {
+            kg[i] = kg0[order[i]];
+            sum_slot[i] = sum0[order[i]];
+            gid[i] = gid0[order[i]];
+        }
+    }
     const auto sweeps = plan_sweeps(kg, 0, kg.size(), nb, RB);
     std::vector<RawOp> raw;
     std::vector<cplx> rpool;
@@ -1573,6 +1657,7 @@ static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGat
         }
         const int RB = qs::kRegBits;
         dp.rb = RB;
+        order_for_sweeps(&kg, dp.gate_off, RB);
         auto swp = plan_sweeps(kg, dp.gate_off, kg.size(), C + dp.j, RB);
         const size_t op0 = ops.size();
         std::vector<RawOp> raw;
@@ -3810,6 +3895,7 @@ qs_status qs_dense_apply_gates(qs_dense *h, const qs_gate *gates, size_t count) 
         p.tile.assign(t.begin(), t.end());
         const size_t g0 = kg.size();
         for (uint32_t gi : p.gates) kg.push_back(to_kgate(cg[gi], p.tile, C));
+        order_for_sweeps(&kg, g0, RB);
         auto swp = plan_sweeps(kg, g0, kg.size(), C + (int)p.tile.size(), RB);
         const size_t op0 = ops.size();
         std::vector<RawOp> raw;

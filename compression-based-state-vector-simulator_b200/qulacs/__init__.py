@@ -665,7 +665,7 @@ class CompressedQuantumState:
         out = np.empty(max(n, 1), dtype=np.uint64)
         self._check(_n.lib().qs_sample_blockwise(self._h, n, int(random_seed) & 0xFFFFFFFF,
                                                  out.ctypes.data_as(_n.ct.POINTER(_n.ct.c_uint64))))
-        return [int(x) for x in out[:n]]
+        return out[:n].tolist()
 
     def __repr__(self):
         return f"CompressedQuantumState(qubits={self._n}, block_size={self._B})"

@@ -96,6 +96,11 @@ class QuantumGateBase:
     def get_matrix(self) -> np.ndarray:
         return self._matrix.copy()
 
+    def _matrix_entries(self) -> List[float]:
+        """get_matrix() as interleaved doubles, row by row."""
+        m = self._matrix if type(self).get_matrix is QuantumGateBase.get_matrix else self.get_matrix()
+        return np.ascontiguousarray(m, dtype=np.complex128).reshape(-1).view(np.float64).tolist()
+
     def get_property_value(self) -> int:
         return self._gate_property
 
@@ -185,6 +190,17 @@ class ParametricRotationGate(QuantumGateBase):
 
     def get_matrix(self) -> np.ndarray:
         return _rotation_matrix(self._axis, self._angle)
+
+    def _matrix_entries(self) -> List[float]:
+        if type(self).get_matrix is not ParametricRotationGate.get_matrix:
+            return super()._matrix_entries()
+        # the entries of _rotation_matrix without an array
+        c, s = math.cos(self._angle / 2), math.sin(self._angle / 2)
+        if self._axis == "X":
+            return [c, 0.0, 0.0, s, 0.0, s, c, 0.0]
+        if self._axis == "Y":
+            return [c, 0.0, s, 0.0, -s, 0.0, c, 0.0]
+        return [c, s, 0.0, 0.0, 0.0, 0.0, c, -s]
 
     @property
     def axis(self) -> str:

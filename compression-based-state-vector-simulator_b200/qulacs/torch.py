@@ -33,6 +33,17 @@ def _masks_arrays(xs, zs):
     return xa, za
 
 
+def _inverse_gate_array(gates):
+    """The packed inverses of gates.  Every gate class of this package inverts
+    to its conjugate transpose (a rotation's entries at -theta are exactly
+    those), taken for all of them at once; a class with a get_inverse of its
+    own is asked."""
+    from ._gates import QuantumGateBase
+    if all(type(g).get_inverse is QuantumGateBase.get_inverse for g in gates):
+        return _n.make_gate_array(gates, inverse=True)
+    return _n.make_gate_array([g.get_inverse() for g in gates])
+
+
 def apply_observable(out: QuantumState, state: QuantumState, observable: Observable) -> None:
     """out := H state (Observable.apply_to_state of the reference)."""
     xs, zs, nys, coefs = observable.term_masks()
@@ -60,7 +71,7 @@ def energy_and_gradient(circuit, observable: Observable, dtype="complex128"):
     back, slots, gx, gz, gny = [], [], [], [], []
     for k in reversed(range(len(gates))):
         g = gates[k]
-        back.append(g.get_inverse())
+        back.append(g)
         if k in slot_of:
             xm, zm, ny = g.generator_masks()
             slots.append(slot_of[k])
@@ -73,7 +84,7 @@ def energy_and_gradient(circuit, observable: Observable, dtype="complex128"):
             gz.append(0)
             gny.append(0)
     nslots = len(param_pos)
-    arr = _n.make_gate_array(back)
+    arr = _inverse_gate_array(back)
     sl = np.ascontiguousarray(np.asarray(slots, dtype=np.int32))
     xa, za = _masks_arrays(gx, gz)
     out = np.zeros(2 * max(1, nslots), dtype=np.float64)
