@@ -1118,7 +1118,7 @@ __global__ void __launch_bounds__(PassShape<R>::kThreads, PassShape<R>::kCtas)
 // ------------------------------------------------------------ staged pass kernel
 // The same fused pass as pass_kernel, restructured so that no global-memory
 // latency sits on a tile's critical path:
-//   * persistent CTAs of kStagedThreads threads walk their tiles in order;
+//   * persistent CTAs (one per SM) walk their tiles in order;
 //     while a CTA works on tile t, the compressed payload of its next tile is
 //     already streaming into a shared-memory double buffer with 1-D bulk
 //     asynchronous copies (cp.async.bulk, one per chunk, completion counted
@@ -1130,7 +1130,10 @@ __global__ void __launch_bounds__(PassShape<R>::kThreads, PassShape<R>::kCtas)
 //     tile's output reservation.
 // Decode, sweeps, quantisation, reservation and packing are pass_kernel's.
 // The copies read this GPU's own memory only (no cluster multicast).
-constexpr int kStagedThreads = 256;
+// Threads of a staged CTA (one per SM): complex64 fits 16 warps, the complex128
+// dense gate holds 2^k amplitudes a thread and needs the registers of 8.
+template <typename R>
+constexpr int kStagedThreads = sizeof(R) == 8 ? 256 : 512;
 // Blocks whose activity / stored bits are kept in shared memory (two bitmasks
 // of this many bits); passes over more blocks read them from global memory.
 constexpr uint32_t kMaxSmemBlocks = 1u << 16;
@@ -1207,7 +1210,7 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
 // Shared-memory layout of staged_pass_kernel (byte offsets; every region
 // 128-byte aligned).
 struct StagedLayout {
-    size_t tile, buf0, buf1, hdr0, hdr1, poff0, poff1, base, width, nz, off, act, sto;
+    size_t tile, buf0, buf1, hdr0, hdr1, poff0, poff1, act, sto;
     size_t dense_a, dense_b, dense_dep;  // dense k-qubit passes only
     size_t total;
 };
@@ -1236,10 +1239,6 @@ __host__ __device__ inline StagedLayout staged_layout(bool f64, int C, int j, ui
     L.hdr1 = o;  o += align128(sizeof(ChunkMeta) * nch);
     L.poff0 = o; o += align128(4 * nch);
     L.poff1 = o; o += align128(4 * nch);
-    L.base = o;  o += align128(4 * nch);
-    L.width = o; o += align128(4 * nch);
-    L.nz = o;    o += align128(4 * nch);
-    L.off = o;   o += align128(8 * nch);
     L.act = o;   o += align128(4 * (size_t)mask_words);
     L.sto = o;   o += align128(4 * (size_t)mask_words);
     if (dense_k > 0) {
@@ -1354,11 +1353,13 @@ __device__ bool tile_dense_k_tc(float2 *tile, int nb, int k, const int32_t *dep,
     float *ahi = aop, *alo = aop + half;
     const float *bhi = bop, *blo = bop + (size_t)Kp * Kp;
     // stage the tile as A = X^T (row o: Re x then Im x), tf32 hi and lo
-    for (int o = threadIdx.x; o < rows; o += blockDim.x) {
+    // (two threads a row, half of its patterns each)
+    for (int w = threadIdx.x; w < 2 * rows; w += blockDim.x) {
+        const int o = w & (rows - 1), half_k = (w >> (nb - k)) * (K / 2);
         const uint32_t base = dense_row_base((uint32_t)o, gmask, nb);
         const int blk = o >> 7, m = o & 127;
         const size_t boff = (size_t)blk * 128 * Kp * 4;
-        for (int r4 = 0; r4 < K; r4 += 4) {
+        for (int r4 = half_k; r4 < half_k + K / 2; r4 += 4) {
             float re[4], im[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -1454,15 +1455,13 @@ __device__ void tile_dense_k_f64(double2 *tile, int nb, int k, const int32_t *de
 // (tile_dense_k_tc / tile_dense_k_f64) instead of the register sweeps.
 // kC, kJ: compile-time chunk log2 and tile qubits (0: from the args).
 template <typename R, bool kCodes, bool kDense, int kC, int kJ>
-__global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const PassArgs a) {
+__global__ void __launch_bounds__(kStagedThreads<R>, 1) staged_pass_kernel(const PassArgs a) {
     using T = typename Cplx<R>::T;
     extern __shared__ __align__(128) unsigned char staged_smem[];
     unsigned char *smem = staged_smem;
     __shared__ __align__(8) uint64_t s_bar[2];
     __shared__ __align__(8) uint64_t s_mma;   // dense complex64: MMA completion
     __shared__ uint32_t s_tmem;               // dense complex64: TMEM base address
-    __shared__ unsigned long long s_tile_off, s_next, s_slab_end;
-    __shared__ int s_flag;
     __shared__ int32_t s_tq[kMaxTileQubits];
     __shared__ int8_t s_oq[kMaxOuterSel];
 
@@ -1470,6 +1469,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
     const int nchunks = 1 << j;
     const int ncomp = 2 << C;
     const int per_lane = ncomp >> 5;
+    constexpr int kPL = kC ? (2 << kC) / 32 : 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int blk_shift = a.B - C;
     const uint32_t nblk = 1u << (a.n - a.B);
@@ -1483,18 +1483,12 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
     auto buf = [&](int s) { return reinterpret_cast<uint32_t *>(smem + Ly.buf0 + (size_t)s * (Ly.buf1 - Ly.buf0)); };
     auto hdr = [&](int s) { return reinterpret_cast<ChunkMeta *>(smem + Ly.hdr0 + (size_t)s * (Ly.hdr1 - Ly.hdr0)); };
     auto poff = [&](int s) { return reinterpret_cast<uint32_t *>(smem + Ly.poff0 + (size_t)s * (Ly.poff1 - Ly.poff0)); };
-    int32_t *s_base = reinterpret_cast<int32_t *>(smem + Ly.base);
-    uint32_t *s_width = reinterpret_cast<uint32_t *>(smem + Ly.width);
-    uint32_t *s_nz = reinterpret_cast<uint32_t *>(smem + Ly.nz);
-    unsigned long long *s_off = reinterpret_cast<unsigned long long *>(smem + Ly.off);
     uint32_t *s_act = reinterpret_cast<uint32_t *>(smem + Ly.act);
     uint32_t *s_sto = reinterpret_cast<uint32_t *>(smem + Ly.sto);
 
     if (threadIdx.x < kMaxTileQubits) s_tq[threadIdx.x] = a.tq[threadIdx.x];
     if (threadIdx.x < kMaxOuterSel) s_oq[threadIdx.x] = a.outer_q[threadIdx.x];
     if (threadIdx.x == 0) {
-        s_next = 0;
-        s_slab_end = 0;
         mbar_init(&s_bar[0], 1);
         mbar_init(&s_bar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -1608,6 +1602,8 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
         }
     };
 
+    const unsigned long long slab = a.slab / nwarps / 128 * 128;  // per warp
+    WarpArena wa;
     unsigned long long rd = 0, wr = 0, ntiles = 0;
     uint32_t phase = 0u;    // bit s: parity of the next phase of s_bar[s]
     uint32_t pending = 0u;  // bit s: a payload fill of buf(s) not yet waited for
@@ -1649,8 +1645,11 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
         // ---- decode this tile's chunks from buf(slot) into the value tile
         for (int c = warp; c < nchunks; c += nwarps) {
             const ChunkMeta md = hdr(slot)[c];
-            unpack_chunk<R, TileSlot<R>, kCodes>(md, per_lane, a.codec, reinterpret_cast<R *>(tile),
-                                                 buf(slot) + (poff(slot)[c] >> 2), lane, TileSlot<R>{c << C});
+            const PairLanes<kPL> pl(per_lane, lane);
+            T *const dst = tile + pos<R>(c << C) + pos<R>(16 * pl.i0) + pos<R>(pl.k);
+            constexpr int kStep = 16 + (16 >> Layout<R>::S1);
+            decode_pairs<R, kCodes, kPL, false>(md, per_lane, a.codec, buf(slot) + (poff(slot)[c] >> 2), lane,
+                                                [&](int i, T v) { dst[i * kStep] = v; });
             if (lane == 0) {
                 const uint64_t chunk = chunk_base | deposit_bits((uint32_t)c, s_tq, j);
                 if (!a.first_pass || block_stored(chunk >> blk_shift))
@@ -1688,79 +1687,21 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
             }
         }
 
-        // ---- quantise (codes replace values in shared memory)
-        for (int c = warp; c < nchunks; c += nwarps) {
-            R *comp = reinterpret_cast<R *>(tile + pos<R>(c << C));
-            int32_t base;
-            uint32_t width;
-            bool nz;
-            quantize_chunk<R, TileSlot<R>, kCodes>(reinterpret_cast<R *>(tile), per_lane, a.codec, a.exact_zero != 0,
-                                                   lane, &base, &width, &nz, TileSlot<R>{c << C},
-                                                   reinterpret_cast<int32_t *>(comp));
-            if (lane == 0) {
-                s_base[c] = base;
-                s_width[c] = width;
-                s_nz[c] = nz ? 1u : 0u;
-            }
-        }
-        __syncthreads();
+        // an arena that overflowed (here or in another CTA) ends the pass
+        if (__syncthreads_or(err_seen)) break;
 
-        // ---- reserve the tile's output bytes (warp 0 scans the chunk sizes)
-        if (warp == 0) {
-            const int per = (nchunks + 31) >> 5;
-            const int c0 = lane * per;
-            unsigned long long mine = 0;
-            for (int c = c0; c < c0 + per && c < nchunks; ++c) mine += payload_bytes(C, s_width[c]);
-            unsigned long long incl = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long t2 = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t2;
-            }
-            unsigned long long run = incl - mine;
-            for (int c = c0; c < c0 + per && c < nchunks; ++c) {
-                s_off[c] = run;
-                run += payload_bytes(C, s_width[c]);
-            }
-            const unsigned long long total = __shfl_sync(0xffffffffu, incl, 31);
-            if (lane == 0) {
-                unsigned long long off = s_next;
-                s_flag = err_seen;
-                if (!err_seen && (a.slab == 0 || off + total > s_slab_end)) {
-                    const unsigned long long want = total > a.slab ? total : a.slab;
-                    off = atomicAdd(a.bump, want);
-                    if (off + want > a.capacity) {
-                        atomicExch(a.error, 1);
-                        s_flag = 1;
-                    }
-                    s_slab_end = off + want;
-                }
-                s_tile_off = off;
-                s_next = off + total;
-                if (!s_flag) wr += total + (unsigned long long)nchunks * sizeof(ChunkMeta);
-            }
-        }
-        __syncthreads();
-        if (s_flag) break;
-
-        // ---- pack and store
+        // ---- quantise, reserve and pack, chunk by chunk
         for (int c = warp; c < nchunks; c += nwarps) {
             const uint64_t chunk = apply_perm(a.perm, chunk_base | deposit_bits((uint32_t)c, s_tq, j));
-            const int32_t *codes = reinterpret_cast<const int32_t *>(tile + pos<R>(c << C));
-            const unsigned long long off = s_tile_off + s_off[c];
-            const uint32_t w = s_width[c];
-            pack_chunk(codes, per_lane, s_base[c], w, a.arena_out + (off >> 2), lane);
-            if (lane == 0) {
-                ChunkMeta md;
-                md.offset = off;
-                md.base = s_base[c];
-                md.width = w;
-                a.meta_out[chunk] = md;
-                if (a.final_pass) {
-                    const uint64_t blk = chunk >> blk_shift;
-                    if (s_nz[c]) atomicOr(&a.block_nz[blk], 1u);
-                    atomicAdd(&a.block_bytes[blk], (unsigned long long)(payload_bytes(C, w) + sizeof(ChunkMeta)));
-                }
+            bool nz;
+            const uint32_t bytes = encode_chunk<R, kCodes, kPL>(tile + pos<R>(c << C), per_lane, C, a.codec,
+                                                                a.exact_zero != 0, lane, wa, slab, a.bump, a.capacity,
+                                                                a.error, a.arena_out, a.meta_out + chunk, &nz);
+            wr += bytes + sizeof(ChunkMeta);
+            if (a.final_pass && lane == 0) {
+                const uint64_t blk = chunk >> blk_shift;
+                if (nz) atomicOr(&a.block_nz[blk], 1u);
+                atomicAdd(&a.block_bytes[blk], (unsigned long long)(bytes + sizeof(ChunkMeta)));
             }
         }
         cur = nxt;
@@ -1783,10 +1724,8 @@ __global__ void __launch_bounds__(kStagedThreads, 1) staged_pass_kernel(const Pa
                          : "memory");
     }
     if (rd) atomicAdd(&a.stats[0], rd);
-    if (threadIdx.x == 0) {
-        if (wr) atomicAdd(&a.stats[1], wr);
-        if (ntiles) atomicAdd(&a.stats[2], ntiles);
-    }
+    if (lane == 0 && wr) atomicAdd(&a.stats[1], wr);
+    if (threadIdx.x == 0 && ntiles) atomicAdd(&a.stats[2], ntiles);
 }
 
 // ------------------------------------------------------------ header permutation pass
@@ -3270,8 +3209,8 @@ static cudaError_t launch_staged_kc(const PassArgs &a, cudaStream_t s) {
     cudaError_t e = ensure_dyn_smem(staged_pass_kernel<R, kCodes, kDense, kC, kJ>, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, staged_pass_kernel<R, kCodes, kDense, kC, kJ>, kStagedThreads,
-                                                      smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, staged_pass_kernel<R, kCodes, kDense, kC, kJ>,
+                                                      kStagedThreads<R>, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     uint64_t grid = (uint64_t)per_sm * sm_count();
@@ -3281,7 +3220,7 @@ static cudaError_t launch_staged_kc(const PassArgs &a, cudaStream_t s) {
     const char *env = std::getenv("QOMPSIM_SLAB_BYTES");
     const uint64_t slab = env ? (uint64_t)std::strtoull(env, nullptr, 10) : (uint64_t)kArenaSlabBytes;
     b.slab = (slab && a.capacity / grid >= 8 * slab) ? (slab + 127) / 128 * 128 : 0;
-    staged_pass_kernel<R, kCodes, kDense, kC, kJ><<<(unsigned)grid, kStagedThreads, smem, s>>>(b);
+    staged_pass_kernel<R, kCodes, kDense, kC, kJ><<<(unsigned)grid, kStagedThreads<R>, smem, s>>>(b);
     return cudaGetLastError();
 }
 
