@@ -1211,6 +1211,8 @@ struct qs_state {
         bool code_moves;      // tile pass whose ops only move amplitudes (X / SWAP)
         qs::ChunkPerm perm;   // where the pass stores each chunk
         std::shared_ptr<const qs::PassProgram> prog;  // the pass's program when it fits one
+        bool shuffle;         // the tile's bits are stored in another order
+        int8_t src_bit[qs::kMaxTileLog2];
     };
     qs::Sweep *sweeps_dev = nullptr;
     qs::ROp *ops_dev = nullptr;
@@ -1594,6 +1596,182 @@ static void make_block_groups(qs_state *h) {
 
 // The device passes of every stage as host data: h->passes plus the op
 // records, sweeps and matrix pool they index.  Host code only.
+// Passes that change the order of the qubits as they go.  A chunk fixes its C
+// lowest qubits, so a tile holds those and jmax others, and a pass that starts
+// from the register's own order spends C of its tile on qubits 0..C-1 whether or
+// not they have gates left.  But a pass may write its tile with any C of the
+// tile's qubits as the chunk qubits of the next pass: the next tile then holds C
+// qubits of this one, chosen by what is still to do, and jmax new ones.  On a
+// chain of neighbours a tile so moves along the register jmax qubits at a time
+// and applies as many layers as its width allows, instead of one or two layers
+// a pass.  The order is put back by the last pass (chunk bits by its chunk
+// permutation), after passes that only move codes when the chunk qubits 0..C-1
+// are not all in its tile.  Only for sequences in which every block is stored:
+// blocks and groups mean nothing in between.
+struct LayoutPass {
+    std::vector<int> tile;         // tile positions >= C, ascending
+    std::vector<CGate> gates;      // on positions
+    std::vector<uint32_t> ids;     // their indices in the sequence
+    std::vector<int> src;          // output tile bit b comes from tile bit src[b]
+};
+
+// False when the sequence has no such plan (a gate that no tile holds).
+// *restore: chunk bit moves after the last pass, from positions to qubits.
+static bool plan_layout_passes(const std::vector<CGate> &sg, int n, int C, int jmax, size_t max_passes,
+                        std::vector<LayoutPass> *out, std::vector<int> *restore) {
+    const int cap = C + jmax;
+    const size_t G = sg.size();
+    if (n < cap || n > 63) return false;
+    std::vector<uint64_t> mix(G, 0), non(G, 0);
+    for (size_t i = 0; i < G; ++i)
+        for (int b = 0; b < sg[i].nq; ++b) (sg[i].mix[b] ? mix[i] : non[i]) |= 1ull << sg[i].q[b];
+    // dependencies as in plan_passes_dag
+    std::vector<std::vector<uint32_t>> succ(G);
+    std::vector<int> indeg(G, 0);
+    {
+        std::vector<int> last_mix(n, -1);
+        std::vector<std::vector<uint32_t>> users(n);
+        for (size_t i = 0; i < G; ++i) {
+            std::set<uint32_t> preds;
+            for (int b = 0; b < sg[i].nq; ++b) {
+                const int q = sg[i].q[b];
+                if (last_mix[q] >= 0) preds.insert((uint32_t)last_mix[q]);
+                if (sg[i].mix[b]) {
+                    preds.insert(users[q].begin(), users[q].end());
+                    last_mix[q] = (int)i;
+                    users[q].clear();
+                } else {
+                    users[q].push_back((uint32_t)i);
+                }
+            }
+            for (uint32_t p : preds) {
+                succ[p].push_back((uint32_t)i);
+                ++indeg[i];
+            }
+        }
+    }
+    const uint64_t low = (1ull << C) - 1;
+    std::set<uint32_t> ready;
+    for (size_t i = 0; i < G; ++i)
+        if (indeg[i] == 0) ready.insert((uint32_t)i);
+    std::vector<char> placed(G, 0);
+    struct Step {
+        uint64_t lo, tile;                // chunk qubits and tile qubits of the pass
+        std::vector<uint32_t> ids;
+    };
+    std::vector<Step> steps;
+    uint64_t carried = low;               // qubits the next chunk can be made of
+    size_t left = G;
+    // how soon a qubit is wanted again: its first unplaced gate, then the
+    // chunk qubits of the final order
+    auto wanted = [&](int q) -> size_t {
+        for (size_t i = 0; i < G; ++i)
+            if (!placed[i] && ((mix[i] >> q) & 1)) return i;
+        return q < C ? G : G + 1;
+    };
+    while (left > 0 || (carried & low) != low) {
+        if (steps.size() >= max_passes) return false;  // not better than the fixed order
+        Step st;
+        uint64_t need = 0, sel = 0;
+        if (left > 0) {
+            bool grew = true;
+            while (grew) {
+                grew = false;
+                for (uint32_t i : ready) {
+                    const uint64_t nn = need | mix[i], ns = sel | non[i];
+                    if (__builtin_popcountll(nn) > cap || __builtin_popcountll(nn & ~carried) > jmax ||
+                        __builtin_popcountll(ns & ~nn) > qs::kMaxOuterSel)
+                        continue;
+                    need = nn;
+                    sel = ns;
+                    st.ids.push_back(i);
+                    placed[i] = 1;
+                    --left;
+                    ready.erase(i);
+                    for (uint32_t sx : succ[i])
+                        if (--indeg[sx] == 0) ready.insert(sx);
+                    grew = true;
+                    break;
+                }
+            }
+            if (st.ids.empty()) return false;
+        } else {
+            // only the order is left: bring in as many of the chunk qubits as fit
+            need = carried & low;
+            for (int q = 0; q < C; ++q)
+                if (!((need >> q) & 1) && __builtin_popcountll(need & ~carried) < jmax) need |= 1ull << q;
+        }
+        std::vector<std::pair<size_t, int>> by_want;
+        for (int q = 0; q < n; ++q) by_want.push_back({wanted(q), q});
+        std::sort(by_want.begin(), by_want.end());
+        // chunk qubits: needed ones of the carried, then those wanted soonest
+        auto take = [&](uint64_t from, int size, uint64_t *set) {
+            for (const auto &w : by_want)
+                if (__builtin_popcountll(*set) < size && ((from >> w.second) & 1)) *set |= 1ull << w.second;
+        };
+        st.lo = 0;
+        take(need & carried, C, &st.lo);
+        take(carried, C, &st.lo);
+        st.tile = st.lo | need;
+        if (left == 0) take(low, cap, &st.tile);
+        take(~0ull >> (64 - n), cap, &st.tile);
+        carried = st.tile;
+        steps.push_back(st);
+    }
+    // positions
+    std::vector<int> at(n), lg(n);  // position of a qubit, qubit at a position
+    for (int q = 0; q < n; ++q) at[q] = lg[q] = q;
+    out->clear();
+    for (size_t p = 0; p < steps.size(); ++p) {
+        const Step &st = steps[p];
+        LayoutPass lp;
+        for (int q = 0; q < n; ++q)
+            if (((st.tile >> q) & 1) && at[q] >= C) lp.tile.push_back(at[q]);
+        std::sort(lp.tile.begin(), lp.tile.end());
+        std::vector<int> slot;  // position of each tile bit
+        for (int b = 0; b < C; ++b) slot.push_back(b);
+        slot.insert(slot.end(), lp.tile.begin(), lp.tile.end());
+        for (uint32_t i : st.ids) {
+            CGate o = sg[i];
+            int order[2] = {0, 0};
+            for (int b = 0; b < o.nq; ++b) order[b] = at[sg[i].q[b]];
+            if (o.nq == 2) reorder_ascending(2, order, sg[i].m, o.q, o.m);
+            else o.q[0] = order[0];
+            compute_mixing(&o);
+            lp.gates.push_back(o);
+            lp.ids.push_back(i);
+        }
+        // the next pass's chunk qubits go to the C lowest positions (a qubit
+        // already there keeps its place), the tile's others to the tile's
+        // upper positions; at the end qubit b to position b
+        const bool last = p + 1 == steps.size();
+        const uint64_t next_lo = last ? low : steps[p + 1].lo;
+        std::vector<int> now(slot.size(), -1);
+        std::vector<int> rest_lo, rest_hi;
+        for (size_t b = 0; b < slot.size(); ++b) {
+            const int q = lg[slot[b]];
+            const bool to_lo = (next_lo >> q) & 1;
+            if (last && to_lo) now[q] = q;
+            else if (to_lo == (b < (size_t)C)) now[b] = q;
+            else (to_lo ? rest_lo : rest_hi).push_back(q);
+        }
+        for (size_t b = 0, l = 0, h = 0; b < slot.size(); ++b)
+            if (now[b] < 0) now[b] = b < (size_t)C ? rest_lo[l++] : rest_hi[h++];
+        lp.src.resize(slot.size());
+        for (size_t b = 0; b < slot.size(); ++b)
+            for (size_t t = 0; t < slot.size(); ++t)
+                if (lg[slot[t]] == now[b]) lp.src[b] = (int)t;
+        for (size_t b = 0; b < slot.size(); ++b) {
+            lg[slot[b]] = now[b];
+            at[now[b]] = slot[b];
+        }
+        out->push_back(std::move(lp));
+    }
+    restore->resize(n - C);
+    for (int s = 0; s < n - C; ++s) (*restore)[s] = lg[s + C] - C;
+    return true;
+}
+
 struct HostPlan {
     std::vector<qs::KGate> kg;
     std::vector<qs::Sweep> sw;
@@ -1606,9 +1784,12 @@ struct HostPlan {
 // their ops, sweeps and matrices in *plan.  A sequence of chunk permutations
 // only becomes one header pass.  *last_gate (when given) receives, per pass,
 // the number k such that gates sg[0..k) have all been applied once the pass
-// is done (passes may take commuting gates out of order).
+// is done (passes may take commuting gates out of order).  layout: every block
+// is stored, so the passes may change the order of the qubits as they go
+// (plan_layout_passes) when that takes fewer of them.
 static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGate> &sg, const HostPerm &P,
-                             HostPlan *plan, std::vector<qs_state::DevPass> *out, std::vector<size_t> *last_gate) {
+                             HostPlan *plan, std::vector<qs_state::DevPass> *out, std::vector<size_t> *last_gate,
+                             bool layout) {
     const int C = (int)h->C;
     const int jmax = std::min(h->tile_log2 - C, qs::kMaxTileQubits);
     // tiles are padded to the largest size: fewer tiles, each with its fixed
@@ -1634,25 +1815,45 @@ static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGat
     std::vector<char> placed_mark(sg.size(), 0);
     auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, sg, C, jmax, jmin, C, (int)h->B)
                                              : plan_passes(ids, sg, C, jmax, jmin, C, (int)h->B);
-    for (size_t p = 0; p < pl.size(); ++p) {
+    std::vector<LayoutPass> lay;
+    HostPerm Pend = P;
+    if (layout && C == qs::kMaxChunkLog2 && pl.size() > 2 && env_int("QOMPSIM_LAYOUT", 1)) {
+        std::vector<int> restore;
+        if (plan_layout_passes(sg, (int)h->n, C, jmax, pl.size() - 1, &lay, &restore)) {
+            for (size_t s = 0; s < restore.size(); ++s) Pend.dst[s] = P.dst[restore[s]];
+        } else {
+            lay.clear();
+        }
+    }
+    const size_t npass = lay.empty() ? pl.size() : lay.size();
+    for (size_t p = 0; p < npass; ++p) {
+        const std::vector<int> &tile = lay.empty() ? pl[p].tile : lay[p].tile;
+        const std::vector<uint32_t> &pass_ids = lay.empty() ? pl[p].gates : lay[p].ids;
         qs_state::DevPass dp{};
         dp.stage = stage;
-        dp.j = (int)pl[p].tile.size();
+        dp.j = (int)tile.size();
         if (dp.j > qs::kMaxTileQubits) return fail(h, QS_ERR_ARG, "tile plan exceeds the tile size");
-        for (int k = 0; k < dp.j; ++k) dp.tq[k] = pl[p].tile[k] - C;
+        for (int k = 0; k < dp.j; ++k) dp.tq[k] = tile[k] - C;
         dp.gate_off = (uint32_t)kg.size();
-        dp.ngates = (uint32_t)pl[p].gates.size();
+        dp.ngates = (uint32_t)pass_ids.size();
         dp.first = p == 0;
-        dp.final = p + 1 == pl.size();
+        dp.final = p + 1 == npass;
         dp.kind = 0;
-        dp.perm = dp.final ? P.device() : identity_perm();
-        for (uint32_t gi : pl[p].gates) kg.push_back(to_kgate(sg[gi], pl[p].tile, C));
+        dp.perm = dp.final ? Pend.device() : identity_perm();
+        for (size_t k = 0; k < pass_ids.size(); ++k)
+            kg.push_back(to_kgate(lay.empty() ? sg[pass_ids[k]] : lay[p].gates[k], tile, C));
+        for (size_t b = 0; !lay.empty() && b < lay[p].src.size(); ++b) {
+            dp.src_bit[b] = (int8_t)lay[p].src[b];
+            dp.shuffle = dp.shuffle || lay[p].src[b] != (int)b;
+        }
         if (last_gate) {
             // gates of sg applied once this pass is done: every gate below the
             // lowest index not yet placed (passes may take gates out of order)
             size_t upto = last_gate->empty() ? 0 : last_gate->back();
-            for (uint32_t gi : pl[p].gates) placed_mark[gi] = 1;
+            for (uint32_t gi : pass_ids) placed_mark[gi] = 1;
             while (upto < sg.size() && placed_mark[upto]) ++upto;
+            // (a changed order of the qubits is only back after the last pass)
+            if (!lay.empty() && !dp.final) upto = std::min(upto, sg.size() - 1);
             last_gate->push_back(upto);
         }
         const int RB = qs::kRegBits;
@@ -1675,7 +1876,7 @@ static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGat
         dp.op_off = (uint32_t)op0;
         dp.sweep_off = (uint32_t)sw.size();
         // a pass of pure register moves carries codes through the tile
-        dp.code_moves = env_int("QOMPSIM_CODE_MOVES", 1) != 0 && ops.size() > op0;
+        dp.code_moves = env_int("QOMPSIM_CODE_MOVES", 1) != 0 && (ops.size() > op0 || pass_ids.empty());
         for (size_t o = op0; o < ops.size() && dp.code_moves; ++o) {
             const int c = ops[o].code;
             dp.code_moves = (c >= qs::OPC_X && c < qs::OPC_X + 8) || (c >= qs::OPC_SWAP && c < qs::OPC_SWAP + 64);
@@ -1696,8 +1897,8 @@ static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGat
             printf("stage %u pass %zu: j=%d gates=%u sweeps=%zu ops=%zu (scalar %d d2 %d m2 %d d4 %d m4 %d, "
                    "half-diagonal %d, moves %d, selectors %d, outer %d)%s tile=[", stage, p, dp.j, dp.ngates,
                    swp.size(), ops.size() - op0, kinds[0], kinds[1], kinds[2], kinds[3], kinds[4], half, moves,
-                   sel, dp.nouter, dp.final && !P.identity() ? " +perm" : "");
-            for (int t : pl[p].tile) printf(" %d", t);
+                   sel, dp.nouter, dp.shuffle ? " +shuffle" : dp.final && !Pend.identity() ? " +perm" : "");
+            for (int t : tile) printf(" %d", t);
             printf(" ]\n");
         }
         dp.nsweeps = (uint32_t)swp.size();
@@ -1723,7 +1924,7 @@ static qs_status plan_device_passes(qs_state *h, HostPlan *plan) {
         std::vector<CGate> sg;
         HostPerm P((int)(h->n - h->C));
         stage_relabel(h->cgates, h->stages[s], C, permute, &sg, &P);
-        qs_status st = emit_passes(h, s, sg, P, plan, &h->passes, nullptr);
+        qs_status st = emit_passes(h, s, sg, P, plan, &h->passes, nullptr, false);
         if (st != QS_OK) return st;
     }
     return QS_OK;
@@ -1764,7 +1965,7 @@ static qs_status plan_tail_passes(qs_state *h, uint32_t s0, HostPlan *plan, std:
         kept_before[i + 1] = sg.size();
     }
     std::vector<size_t> last_gate;
-    qs_status st = emit_passes(h, s0, sg, P, plan, passes, &last_gate);
+    qs_status st = emit_passes(h, s0, sg, P, plan, passes, &last_gate, true);
     if (st != QS_OK) return st;
     for (size_t k = 0; k < stage_end.size(); ++k) {
         const size_t kept = kept_before[stage_end[k]];  // relabelled gates up to this stage's end
@@ -2072,6 +2273,8 @@ qs_status qs_apply_circuit(qs_state *h) {
         a.meta_out = h->meta[h->mcur ^ 1];
         a.arena_out = h->arena[out];
         a.perm = dp.perm;
+        a.shuffle = dp.shuffle ? 1 : 0;
+        for (int b = 0; b < qs::kMaxTileLog2; ++b) a.src_bit[b] = dp.src_bit[b];
         a.bump = h->counters + out;
         a.capacity = h->capacity;
         a.block_to_group = b2g;

@@ -245,6 +245,8 @@ struct PassArgs {
     int32_t *error;                     // 1 = arena overflow, 2 = a bounded wait for staged payloads gave up
     unsigned long long *stats;          // [0] bytes read [1] bytes written [2] tiles
     ChunkPerm perm;                     // chunk c of the pass is stored as chunk perm(c)
+    int32_t shuffle;                    // 1: the tile is written with its bits in another order (2^8-amplitude
+    int8_t src_bit[kMaxTileLog2];       // chunks): bit b of an output tile index is bit src_bit[b] of the tile
     int32_t nouter;                     // outer selector qubits of the pass
     int8_t outer_q[kMaxOuterSel];       // their global qubit indices (bit nb + i of W)
     DiagSum diag;                       // nterms > 0: multiply by a diagonal Pauli sum after the sweeps

@@ -72,12 +72,13 @@ __device__ __forceinline__ uint64_t deposit_bits(uint32_t c, const int32_t *pos,
 }
 
 // ------------------------------------------------------------ tile layout
-// Element e of a tile lives at shared-memory slot pos(e) = e + (e >> S1): one
-// slot of padding after every 128 bytes, so that a warp whose lanes differ in
-// bits above S1 spreads over the banks.  pos is additive over disjoint bits
-// (pos(a | b) = pos(a) + pos(b)), so a sweep's 16 offsets are sums of four
-// uniform numbers and a lane's components of a chunk lie at compile-time
-// distances from its first one.  (The XOR layout used before cost five
+// Element e of a tile lives at shared-memory slot pos(e) = e + (e >> S1) + (e >>
+// 2 S1) + (e >> 3 S1): padding after every 128 bytes, again after every such
+// group of groups and so on, so that a warp whose lanes differ in any run of
+// bits spreads over the banks.  pos is additive over disjoint bits (pos(a | b) =
+// pos(a) + pos(b)), so a sweep's 16 offsets are sums of four uniform numbers and
+// a lane's components of a chunk lie at compile-time distances from its first
+// one.  (The XOR layout used before cost five
 // instructions a component in the codec and again in every sweep.)
 template <typename R> struct Layout;
 template <> struct Layout<double> { static constexpr int S1 = 3; };
@@ -85,7 +86,8 @@ template <> struct Layout<float> { static constexpr int S1 = 4; };
 
 template <typename R>
 __host__ __device__ __forceinline__ constexpr int pos(int e) {
-    return e + (e >> Layout<R>::S1);
+    constexpr int S = Layout<R>::S1;
+    return e + (e >> S) + (e >> 2 * S) + (e >> 3 * S);
 }
 
 // Bytes of a tile of 2^nb amplitudes.
@@ -792,8 +794,7 @@ __device__ __forceinline__ void unpack_in_place(const ChunkMeta md, int per_lane
     using T = typename Cplx<R>::T;
     const PairLanes<kPL> pl(per_lane, lane);
     T *const dst = chunk_elem0 + pos<R>(16 * pl.i0) + pos<R>(pl.k);
-    constexpr int kStep = 16 + (16 >> Layout<R>::S1);
-    decode_pairs<R, kCodes, kPL, true>(md, per_lane, p, src, lane, [&](int i, T v) { dst[i * kStep] = v; });
+    decode_pairs<R, kCodes, kPL, true>(md, per_lane, p, src, lane, [&](int i, T v) { dst[pos<R>(16 * i)] = v; });
 }
 
 // A warp's chunks gw, gw + nw, ... of [chunk0, chunk0 + nchunks) in turn:
@@ -864,8 +865,15 @@ struct WarpArena {
 // that finds the arena full gets a zero header (the error flag is set).
 // Returns the payload bytes; *nz: some amplitude is not zero (with exact_zero
 // the values are tested, else the codes: code 0 is exactly the value 0).
+// chunk_elem0: the chunk's first element; with sh.on (2^8-amplitude chunks) the
+// slot of the lane's first amplitude, the others at sums of the sh.step.
+struct ShuffleSteps {
+    bool on = false;
+    int step[3];
+};
 template <typename R, bool kCodes, int kPL>
-__device__ __forceinline__ uint32_t encode_chunk(const typename Cplx<R>::T *chunk_elem0, int per_lane, int C,
+__device__ __forceinline__ uint32_t encode_chunk(const typename Cplx<R>::T *chunk_elem0, const ShuffleSteps &sh,
+                                                 int per_lane, int C,
                                                  CodecParams p, bool exact_zero, int lane, WarpArena &wa,
                                                  unsigned long long slab, unsigned long long *bump,
                                                  unsigned long long capacity, int32_t *error,
@@ -873,14 +881,17 @@ __device__ __forceinline__ uint32_t encode_chunk(const typename Cplx<R>::T *chun
     using T = typename Cplx<R>::T;
     const PairLanes<kPL> pl(per_lane, lane);
     constexpr int H = PairLanes<kPL>::H;
-    const T *const src = chunk_elem0 + pos<R>(16 * pl.i0) + pos<R>(pl.k);
-    constexpr int kStep = 16 + (16 >> Layout<R>::S1);
+    const T *const src = sh.on ? chunk_elem0 : chunk_elem0 + pos<R>(16 * pl.i0) + pos<R>(pl.k);
+    auto at = [&](int i) {
+        return sh.on ? ((i & 1) ? sh.step[0] : 0) + ((i & 2) ? sh.step[1] : 0) + ((i & 4) ? sh.step[2] : 0)
+                     : pos<R>(16 * i);
+    };
     int32_t q0[H], q1[H];
     int32_t lo = INT_MAX, hi = INT_MIN;
 #pragma unroll
     for (int i = 0; i < H; ++i) {
         if (i < pl.n) {
-            const T v = src[i * kStep];
+            const T v = src[at(i)];
             q0[i] = kCodes ? value_as_code(v.x) : quantize_hot(v.x, p);
             q1[i] = kCodes ? value_as_code(v.y) : quantize_hot(v.y, p);
             lo = __vimin3_s32(lo, q0[i], q1[i]);
@@ -891,7 +902,7 @@ __device__ __forceinline__ uint32_t encode_chunk(const typename Cplx<R>::T *chun
     hi = __reduce_max_sync(0xffffffffu, hi);
     if (!kCodes && exact_zero) {
         bool any = false;
-        for (int i = 0; i < pl.n; ++i) any |= src[i * kStep].x != R(0) || src[i * kStep].y != R(0);
+        for (int i = 0; i < pl.n; ++i) any |= src[at(i)].x != R(0) || src[at(i)].y != R(0);
         *nz = __any_sync(0xffffffffu, any);
     } else {
         *nz = (lo | hi) != 0;
@@ -991,6 +1002,24 @@ __device__ void tile_diag_sum(typename Cplx<R>::T *tile, int nb, const DiagSum &
     __syncthreads();
 }
 
+// Where a shuffled tile's output elements come from: amplitude bits 0..3 and 7
+// are the lane's (its offset is returned), 4..6 the lane's successive
+// amplitudes (sh.step), the others the chunk's (shuffle_chunk).
+template <typename R>
+__device__ __forceinline__ int shuffle_lane(const PassArgs &a, int lane, ShuffleSteps &sh) {
+    if (!a.shuffle) return 0;
+    sh.on = true;
+    int off = (lane >> 4) ? pos<R>(1 << a.src_bit[7]) : 0;
+    for (int b = 0; b < 3; ++b) sh.step[b] = pos<R>(1 << a.src_bit[4 + b]);
+    for (int b = 0; b < 4; ++b) off += ((lane >> b) & 1) ? pos<R>(1 << a.src_bit[b]) : 0;
+    return off;
+}
+template <typename R>
+__device__ __forceinline__ int shuffle_chunk(const PassArgs &a, int c, int C, int j, int lane_off) {
+    for (int b = 0; b < j; ++b) lane_off += ((c >> b) & 1) ? pos<R>(1 << a.src_bit[C + b]) : 0;
+    return lane_off;
+}
+
 // ------------------------------------------------------------ pass kernel
 // kCodes: every op of the pass only moves amplitudes (X / SWAP register
 // moves, chunk permutations), so the tile holds the quantised codes
@@ -1015,7 +1044,9 @@ struct PassShape {
 
 // Prog: PassProgram (the default geometry), or NoProgram: the ops are read
 // from global memory.
-template <typename R, int RB, bool kCodes, int kC, int kJ, typename Prog>
+// kShuffle: the tile's bits may be stored in another order (a.shuffle); without
+// it a lane's elements lie at compile-time offsets (3 to 7 % faster passes).
+template <typename R, int RB, bool kCodes, int kC, int kJ, typename Prog, bool kShuffle>
 __global__ void __launch_bounds__(PassShape<R>::kThreads, PassShape<R>::kCtas)
     pass_kernel(const __grid_constant__ PassArgs a, const __grid_constant__ Prog prog) {
     using T = typename Cplx<R>::T;
@@ -1049,6 +1080,9 @@ __global__ void __launch_bounds__(PassShape<R>::kThreads, PassShape<R>::kCtas)
     }
     __syncthreads();
     const unsigned long long slab = a.slab / (PassShape<R>::kThreads / 32) / 128 * 128;  // per warp
+    ShuffleSteps sh;
+    int lane_off = 0;
+    if constexpr (kShuffle) lane_off = shuffle_lane<R>(a, lane, sh);
 
     WarpArena wa;
     unsigned long long rd = 0, wr = 0, ntiles = 0;
@@ -1098,7 +1132,8 @@ __global__ void __launch_bounds__(PassShape<R>::kThreads, PassShape<R>::kCtas)
         for (int c = warp; c < nchunks; c += nwarps) {
             const uint64_t chunk = (out_base | s_out[c]) ^ a.perm.flip;
             bool nz;
-            const uint32_t bytes = encode_chunk<R, kCodes, kPL>(tile + pos<R>(c << C), per_lane, C, a.codec,
+            const int first = sh.on ? shuffle_chunk<R>(a, c, C, j, lane_off) : pos<R>(c << C);
+            const uint32_t bytes = encode_chunk<R, kCodes, kPL>(tile + first, sh, per_lane, C, a.codec,
                                                                 a.exact_zero != 0, lane, wa, slab, a.bump, a.capacity,
                                                                 a.error, a.arena_out, a.meta_out + chunk, &nz);
             wr += bytes + sizeof(ChunkMeta);
@@ -1108,7 +1143,9 @@ __global__ void __launch_bounds__(PassShape<R>::kThreads, PassShape<R>::kCtas)
                 atomicAdd(&a.block_bytes[blk], (unsigned long long)(bytes + sizeof(ChunkMeta)));
             }
         }
-        __syncwarp();
+        // a warp's output chunks may come from anywhere in a shuffled tile
+        if (sh.on) __syncthreads();
+        else __syncwarp();
     }
     if (rd) atomicAdd(&a.stats[0], rd);
     if (lane == 0 && wr) atomicAdd(&a.stats[1], wr);
@@ -1455,7 +1492,8 @@ __device__ void tile_dense_k_f64(double2 *tile, int nb, int k, const int32_t *de
 // (tile_dense_k_tc / tile_dense_k_f64) instead of the register sweeps.
 // kC, kJ: compile-time chunk log2 and tile qubits (0: from the args).
 template <typename R, bool kCodes, bool kDense, int kC, int kJ>
-__global__ void __launch_bounds__(kStagedThreads<R>, 1) staged_pass_kernel(const PassArgs a) {
+__global__ void __launch_bounds__(kStagedThreads<R>, 1)
+    staged_pass_kernel(const __grid_constant__ PassArgs a) {
     using T = typename Cplx<R>::T;
     extern __shared__ __align__(128) unsigned char staged_smem[];
     unsigned char *smem = staged_smem;
@@ -1603,6 +1641,8 @@ __global__ void __launch_bounds__(kStagedThreads<R>, 1) staged_pass_kernel(const
     };
 
     const unsigned long long slab = a.slab / nwarps / 128 * 128;  // per warp
+    ShuffleSteps sh;
+    const int lane_off = shuffle_lane<R>(a, lane, sh);
     WarpArena wa;
     unsigned long long rd = 0, wr = 0, ntiles = 0;
     uint32_t phase = 0u;    // bit s: parity of the next phase of s_bar[s]
@@ -1647,9 +1687,8 @@ __global__ void __launch_bounds__(kStagedThreads<R>, 1) staged_pass_kernel(const
             const ChunkMeta md = hdr(slot)[c];
             const PairLanes<kPL> pl(per_lane, lane);
             T *const dst = tile + pos<R>(c << C) + pos<R>(16 * pl.i0) + pos<R>(pl.k);
-            constexpr int kStep = 16 + (16 >> Layout<R>::S1);
             decode_pairs<R, kCodes, kPL, false>(md, per_lane, a.codec, buf(slot) + (poff(slot)[c] >> 2), lane,
-                                                [&](int i, T v) { dst[i * kStep] = v; });
+                                                [&](int i, T v) { dst[pos<R>(16 * i)] = v; });
             if (lane == 0) {
                 const uint64_t chunk = chunk_base | deposit_bits((uint32_t)c, s_tq, j);
                 if (!a.first_pass || block_stored(chunk >> blk_shift))
@@ -1694,7 +1733,8 @@ __global__ void __launch_bounds__(kStagedThreads<R>, 1) staged_pass_kernel(const
         for (int c = warp; c < nchunks; c += nwarps) {
             const uint64_t chunk = apply_perm(a.perm, chunk_base | deposit_bits((uint32_t)c, s_tq, j));
             bool nz;
-            const uint32_t bytes = encode_chunk<R, kCodes, kPL>(tile + pos<R>(c << C), per_lane, C, a.codec,
+            const int first = sh.on ? shuffle_chunk<R>(a, c, C, j, lane_off) : pos<R>(c << C);
+            const uint32_t bytes = encode_chunk<R, kCodes, kPL>(tile + first, sh, per_lane, C, a.codec,
                                                                 a.exact_zero != 0, lane, wa, slab, a.bump, a.capacity,
                                                                 a.error, a.arena_out, a.meta_out + chunk, &nz);
             wr += bytes + sizeof(ChunkMeta);
@@ -1797,9 +1837,13 @@ __global__ void __launch_bounds__(kSweepThreads, 3) dense_pass_kernel(const __gr
         const uint64_t chunk_base = insert_zero_bits(tile_id, s_tq, j);
         T *const st0 = st + (chunk_base << C);
         // every load of the tile in flight at once, straight into shared memory
+        // (pos is additive: the thread's part once, the rest uniform)
 #pragma unroll 4
-        for (int e = threadIdx.x; e < size; e += kSweepThreads)
-            cp_async_elem<sizeof(T)>(&tile[pos<R>(e)], &st0[s_off[e >> C] + (e & cmask)]);
+        for (int e0 = 0; e0 < size; e0 += kSweepThreads) {
+            const int e = e0 + threadIdx.x;
+            if (e < size)
+                cp_async_elem<sizeof(T)>(tile + pos<R>(threadIdx.x) + pos<R>(e0), &st0[s_off[e >> C] + (e & cmask)]);
+        }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
         // the CTA's next tile starts its way into L2 while this one is worked on
@@ -1815,7 +1859,10 @@ __global__ void __launch_bounds__(kSweepThreads, 3) dense_pass_kernel(const __gr
         else
             tile_sweeps<R, RB>(tile, nb, a.sweeps, a.nsweeps, a.ops, reinterpret_cast<const T *>(a.pool), ow);
 #pragma unroll 8
-        for (int e = threadIdx.x; e < size; e += kSweepThreads) st0[s_off[e >> C] + (e & cmask)] = tile[pos<R>(e)];
+        for (int e0 = 0; e0 < size; e0 += kSweepThreads) {
+            const int e = e0 + threadIdx.x;
+            if (e < size) st0[s_off[e >> C] + (e & cmask)] = tile[pos<R>(threadIdx.x) + pos<R>(e0)];
+        }
         __syncthreads();
     }
 }
@@ -2750,10 +2797,11 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
     for (uint64_t tile_id = blockIdx.x; tile_id < a.n_tiles; tile_id += gridDim.x) {
         const uint64_t base_amp = insert_zero_bits(tile_id, s_tq, kJ) << kC;
 #pragma unroll 4
-        for (int e = threadIdx.x; e < size; e += kAdjThreads) {
+        for (int e0 = 0; e0 < size; e0 += kAdjThreads) {
+            const int e = e0 + threadIdx.x, at = pos<R>(threadIdx.x) + pos<R>(e0);
             const uint64_t amp = base_amp + s_off[e >> kC] + (e & cmask);
-            cp_async_elem<sizeof(T)>(&tp[pos<R>(e)], &psi[amp]);
-            cp_async_elem<sizeof(T)>(&tl[pos<R>(e)], &lam[amp]);
+            cp_async_elem<sizeof(T)>(&tp[at], &psi[amp]);
+            cp_async_elem<sizeof(T)>(&tl[at], &lam[amp]);
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
@@ -2835,10 +2883,11 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
             __syncthreads();
         }
 #pragma unroll 4
-        for (int e = threadIdx.x; e < size; e += kAdjThreads) {
+        for (int e0 = 0; e0 < size; e0 += kAdjThreads) {
+            const int e = e0 + threadIdx.x, at = pos<R>(threadIdx.x) + pos<R>(e0);
             const uint64_t amp = base_amp + s_off[e >> kC] + (e & cmask);
-            psi[amp] = tp[pos<R>(e)];
-            lam[amp] = tl[pos<R>(e)];
+            psi[amp] = tp[at];
+            lam[amp] = tl[at];
         }
         __syncthreads();
     }
@@ -3161,14 +3210,14 @@ int sm_count() {
     return g_sm_count;
 }
 
-template <typename R, int RB, bool kCodes, int kC, int kJ, typename Prog>
+template <typename R, int RB, bool kCodes, int kC, int kJ, typename Prog, bool kShuffle>
 static cudaError_t launch_pass_kc(const PassArgs &a, const Prog &prog, cudaStream_t s) {
     const int nb = a.C + a.j;
     const size_t smem = pass_smem_bytes(sizeof(R) == 8, nb, a.j, a.diag.nterms);
-    cudaError_t e = ensure_dyn_smem(pass_kernel<R, RB, kCodes, kC, kJ, Prog>, smem);
+    cudaError_t e = ensure_dyn_smem(pass_kernel<R, RB, kCodes, kC, kJ, Prog, kShuffle>, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<R, RB, kCodes, kC, kJ, Prog>,
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<R, RB, kCodes, kC, kJ, Prog, kShuffle>,
                                                       PassShape<R>::kThreads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
@@ -3181,7 +3230,7 @@ static cudaError_t launch_pass_kc(const PassArgs &a, const Prog &prog, cudaStrea
     const char *env = std::getenv("QOMPSIM_SLAB_BYTES");
     const uint64_t slab = env ? (uint64_t)std::strtoull(env, nullptr, 10) : (uint64_t)kArenaSlabBytes;
     b.slab = (slab && a.capacity / grid >= 8 * slab) ? (slab + 127) / 128 * 128 : 0;
-    pass_kernel<R, RB, kCodes, kC, kJ, Prog><<<(unsigned)grid, PassShape<R>::kThreads, smem, s>>>(b, prog);
+    pass_kernel<R, RB, kCodes, kC, kJ, Prog, kShuffle><<<(unsigned)grid, PassShape<R>::kThreads, smem, s>>>(b, prog);
     return cudaGetLastError();
 }
 
@@ -3196,9 +3245,10 @@ template <typename R, int RB, bool kCodes>
 static cudaError_t launch_pass_t(const PassArgs &a, const PassProgram *prog, cudaStream_t s) {
     constexpr int J = sizeof(R) == 8 ? 4 : 5;
     if (a.C == kMaxChunkLog2 && a.j == J && prog)
-        return launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, J, PassProgram>(a, *prog, s);
-    return a.C == kMaxChunkLog2 ? launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, 0, NoProgram>(a, NoProgram{}, s)
-                                : launch_pass_kc<R, RB, kCodes, 0, 0, NoProgram>(a, NoProgram{}, s);
+        return a.shuffle ? launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, J, PassProgram, true>(a, *prog, s)
+                         : launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, J, PassProgram, false>(a, *prog, s);
+    return a.C == kMaxChunkLog2 ? launch_pass_kc<R, RB, kCodes, kMaxChunkLog2, 0, NoProgram, true>(a, NoProgram{}, s)
+                                : launch_pass_kc<R, RB, kCodes, 0, 0, NoProgram, false>(a, NoProgram{}, s);
 }
 
 template <typename R, bool kCodes, bool kDense, int kC, int kJ>
@@ -3238,6 +3288,14 @@ static cudaError_t launch_staged_t(const PassArgs &a, cudaStream_t s) {
 cudaError_t launch_pass(bool f64, const PassArgs &a, const PassProgram *prog, cudaStream_t s) {
     if (a.rb != kRegBits || a.C + a.j < kRegBits || a.diag.nterms > kMaxDiagTerms) return cudaErrorInvalidValue;
     if (a.code_moves && a.diag.nterms) return cudaErrorInvalidValue;
+    if (a.shuffle) {
+        // a permutation of the tile's bits, 2^8-amplitude chunks
+        uint32_t seen = 0;
+        for (int b = 0; b < a.C + a.j; ++b)
+            if (a.src_bit[b] >= 0 && a.src_bit[b] < a.C + a.j) seen |= 1u << a.src_bit[b];
+        if (a.C != kMaxChunkLog2 || a.dense.k || seen != (1u << (a.C + a.j)) - 1u)
+            return cudaErrorInvalidValue;
+    }
     if (a.dense.k) {
         // one dense k-qubit gate over 2^kDenseTileLog2-amplitude tiles (staged kernel only)
         if (a.dense.k < kMinDenseK || a.dense.k > kMaxDenseK || a.C + a.j != kDenseTileLog2 || a.code_moves ||
