@@ -129,6 +129,9 @@ static_assert(sizeof(KGate) == 288, "KGate layout");
 //             variant * stride), else its entries lie in mats at entry `mat`
 //   variant   ((W >> s1) & m1) + (((W >> s2) & m2) << l1); with kProgSelList
 //             s1 and m1 hold the selector positions as bytes instead
+//   kProgM2C  a two-qubit matrix that is block diagonal in one of its bits: two
+//             2x2 matrices (mats entries 0..3 and 4..7), place bit 3 t + i for
+//             target bit t and the i-th of the other three bits as selector
 //   kProgSum  (two-state passes) OPC_SUM: mat = slot, stride = xs << 4 | zs, the
 //             sign is the parity of W & s1
 // One-hot bits instead of a code: the device tests them one after another, and
@@ -137,7 +140,7 @@ static_assert(sizeof(KGate) == 288, "KGate layout");
 // double precision) after every op.
 constexpr uint32_t kProgScalar = 1, kProgAcc = 2, kProgHalf = 4, kProgHalfPending = 8, kProgDiag = 16, kProgM2 = 32,
                    kProgX = 64, kProgHalf4 = 128, kProgDiag4 = 256, kProgM4 = 512, kProgSwap = 1024,
-                   kProgSum = 2048;
+                   kProgSum = 2048, kProgM2C = 4096;
 constexpr uint32_t kProgVar = 1u << 14, kProgSelList = 1u << 15;
 constexpr int kProgWhere = 16;
 constexpr int kProgOps = 192, kProgSweeps = 32, kProgMatBytes = 8192;
