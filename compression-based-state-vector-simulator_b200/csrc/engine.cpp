@@ -800,6 +800,17 @@ bool finalize_ops(const std::vector<RawOp> &raw, const std::vector<cplx> &rpool,
     return true;
 }
 
+// Exact SWAP of two tile bits.
+bool is_swap(const qs::KGate &g) {
+    if (g.nq != 2 || g.tpos[0] < 0 || g.tpos[1] < 0) return false;
+    for (int y = 0; y < 4; ++y)
+        for (int x = 0; x < 4; ++x) {
+            const int to = y == 1 ? 2 : y == 2 ? 1 : y;
+            if (g.m[2 * (4 * y + x)] != (x == to ? 1.0 : 0.0) || g.m[2 * (4 * y + x) + 1] != 0.0) return false;
+        }
+    return true;
+}
+
 // Class and place bits of an op code; false for codes that no program holds.
 bool program_op(int code, uint32_t *what) {
     struct { int base; uint32_t cls; bool pair; } const kinds[] = {
@@ -1910,6 +1921,28 @@ static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGat
         for (size_t o = op0; o < ops.size() && dp.code_moves; ++o) {
             const int c = ops[o].code;
             dp.code_moves = (c >= qs::OPC_X && c < qs::OPC_X + 8) || (c >= qs::OPC_SWAP && c < qs::OPC_SWAP + 64);
+        }
+        // A pass of SWAPs alone only reorders the tile's bits: the encode reads
+        // them in the other order and no sweep is needed (QFT bit reversal).
+        if (dp.code_moves && C == qs::kMaxChunkLog2 && !pass_ids.empty() && env_int("QOMPSIM_LAYOUT", 1)) {
+            std::vector<int> from(C + dp.j);  // tile bit t holds the pass's input bit from[t]
+            for (size_t t = 0; t < from.size(); ++t) from[t] = (int)t;
+            bool swaps = true;
+            for (size_t g = dp.gate_off; g < kg.size() && swaps; ++g) {
+                swaps = is_swap(kg[g]);
+                if (swaps) std::swap(from[kg[g].tpos[0]], from[kg[g].tpos[1]]);
+            }
+            if (swaps) {
+                int8_t out_bit[qs::kMaxTileLog2];
+                for (size_t b = 0; b < from.size(); ++b)
+                    out_bit[b] = (int8_t)from[lay.empty() ? b : (size_t)lay[p].src[b]];
+                dp.shuffle = false;
+                for (size_t b = 0; b < from.size(); ++b) {
+                    dp.src_bit[b] = out_bit[b];
+                    dp.shuffle = dp.shuffle || out_bit[b] != (int)b;
+                }
+                swp.clear();
+            }
         }
         if (std::getenv("QOMPSIM_DEBUG_PLAN")) {
             int kinds[5] = {0, 0, 0, 0, 0}, sel = 0, half = 0, moves = 0;
