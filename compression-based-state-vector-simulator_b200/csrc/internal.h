@@ -11,8 +11,9 @@ namespace qs {
 
 // Largest chunk: 2^8 amplitudes = 512 real components = 16 per lane.
 constexpr int kMaxChunkLog2 = 8;
-// Arena space a pass-kernel CTA takes at once (when the arena holds at least
-// eight per CTA), sub-allocated to its tiles without the shared counter.
+// Arena space a pass-kernel CTA may take at once (when the arena holds at least
+// eight per CTA), an equal share for each of its warps, sub-allocated to the
+// warp's chunks without the shared counter.
 constexpr uint64_t kArenaSlabBytes = 256 << 10;
 constexpr int kMinChunkLog2 = 4;
 constexpr int kMaxPerLane = (2 << kMaxChunkLog2) / 32;

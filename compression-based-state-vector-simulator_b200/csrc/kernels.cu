@@ -11,9 +11,9 @@
 // differ exactly in the pass's tile qubits, so every gate of the pass that
 // mixes amplitudes acts inside one tile.  A CTA decodes the tile's chunks
 // into shared memory (one warp per chunk, coalesced 128-byte payload rows),
-// applies the pass's gates in shared memory, re-quantises, reserves output
-// space for the whole tile with one atomicAdd on the arena's bump counter
-// and writes the packed chunks back with coalesced stores.
+// applies the pass's gates in registers and shared memory, and each warp
+// quantises its chunks, packs them into its own slab of the output arena and
+// writes them back with coalesced stores.
 #include <cstdio>
 #include <climits>
 #include <cstdlib>
@@ -572,12 +572,7 @@ struct LinearSlot {
     __device__ __forceinline__ int operator()(int c) const { return c; }
 };
 
-// Component c of the chunk that starts at tile element elem0.
-template <typename R>
-struct TileSlot {
-    int elem0;
-    __device__ __forceinline__ int operator()(int c) const { return 2 * pos<R>(elem0 + (c >> 1)) + (c & 1); }
-};
+// Component c of the chunk that starts at tile element elem0 (XOR layout).
 template <typename R>
 struct XorSlot {
     int elem0, swm;
@@ -628,14 +623,14 @@ __device__ __forceinline__ void cp_async_wait() {
 // Unpack a chunk whose payload is in the warp's staging buffer (the copy
 // complete and visible to the warp): every element is extracted on its own
 // (one funnel shift); a lane reads only its own words.
-template <typename R, typename Slot = LinearSlot, bool kCodes = false>
+template <typename R, typename Slot = LinearSlot>
 __device__ __forceinline__ void unpack_chunk(const ChunkMeta md, int per_lane, CodecParams p, R *comp,
                                              const uint32_t *wstage, int lane, Slot slot = Slot()) {
     // a width above 32 never comes from a pass or a checked import; clamped so
     // that no header can make the unpack read past its chunk's staged rows
     const uint32_t w = md.width > 32 ? 32u : md.width;
     if (w == 0) {
-        const R v = kCodes ? code_as_value(md.base, R()) : dequantize_hot(md.base, p, R());
+        const R v = dequantize_hot(md.base, p, R());
         for (int i = 0; i < per_lane; ++i) comp[slot(lane + 32 * i)] = v;
         return;
     }
@@ -646,14 +641,14 @@ __device__ __forceinline__ void unpack_chunk(const ChunkMeta md, int per_lane, C
             const uint32_t bit = (uint32_t)i * w, r = bit >> 5;
             const uint32_t u = __funnelshift_r(wstage[r * 32 + lane], wstage[(r + 1) * 32 + lane], bit & 31) & mask;
             const int32_t code = (int32_t)((uint32_t)md.base + u);
-            comp[slot(lane + 32 * i)] = kCodes ? code_as_value(code, R()) : dequantize_hot(code, p, R());
+            comp[slot(lane + 32 * i)] = dequantize_hot(code, p, R());
         }
     }
 }
 
 // Per-warp decode of one chunk: copy its payload into the warp's staging
 // area (one round trip to memory), then unpack it.
-template <typename R, typename Slot = LinearSlot, bool kCodes = false>
+template <typename R, typename Slot = LinearSlot>
 __device__ __forceinline__ void decode_chunk(const uint32_t *__restrict__ arena, const ChunkMeta md,
                                              int per_lane, CodecParams p, R *comp, uint32_t *wstage,
                                              int lane, Slot slot = Slot()) {
@@ -662,13 +657,13 @@ __device__ __forceinline__ void decode_chunk(const uint32_t *__restrict__ arena,
         cp_async_wait<0>();
         __syncwarp();
     }
-    unpack_chunk<R, Slot, kCodes>(md, per_lane, p, comp, wstage, lane, slot);
+    unpack_chunk<R, Slot>(md, per_lane, p, comp, wstage, lane, slot);
 }
 
 // Per-warp quantisation of one chunk held in comp[]: codes overwrite the
 // chunk's own shared memory as int32.  Returns
 // base/width/non-zero flag (valid in every lane).
-template <typename R, typename Slot = LinearSlot, bool kCodes = false>
+template <typename R, typename Slot = LinearSlot>
 __device__ __forceinline__ void quantize_chunk(R *comp, int per_lane, CodecParams p, bool exact_zero,
                                                int lane, int32_t *base_out, uint32_t *width_out,
                                                bool *nz_out, Slot slot = Slot(), int32_t *codes = nullptr) {
@@ -689,12 +684,12 @@ __device__ __forceinline__ void quantize_chunk(R *comp, int per_lane, CodecParam
 #pragma unroll
         for (int i = 0; i < H; ++i) {
             if (h * H + i < per_lane) {
-                const int32_t q = kCodes ? value_as_code(v[i]) : quantize_hot(v[i], p);
+                const int32_t q = quantize_hot(v[i], p);
                 codes[lane + 32 * (h * H + i)] = q;
                 lo = min(lo, q);
                 hi = max(hi, q);
                 // code 0 is exactly the value 0
-                nz |= (exact_zero && !kCodes) ? (v[i] != R(0)) : (q != 0);
+                nz |= exact_zero ? (v[i] != R(0)) : (q != 0);
             }
         }
         __syncwarp();
@@ -2532,15 +2527,15 @@ __device__ void dual_tile_sweeps(typename Cplx<R>::T *tA, typename Cplx<R>::T *t
                                  int nsweeps, const ROp *__restrict__ ops, const typename Cplx<R>::T *__restrict__ pool,
                                  uint32_t ow, double *s_acc, int lane);
 
-// kC, kJ: the chunk and tile-qubit counts as compile-time constants (0 = read
-// them from the launch arguments).
-template <typename R, int kC, int kJ>
+// The backward pass in any geometry and for any op list (adjoint_prog_kernel
+// takes the default geometry's programs).
+template <typename R>
 __global__ void __launch_bounds__(kAdjThreads, 2) adjoint_pass_kernel(const AdjPassArgs a) {
     using T = typename Cplx<R>::T;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double s_acc[2 * kMaxAdjSlots];
     __shared__ int32_t s_tq[kMaxTileQubits];
-    const int C = kC ? kC : a.C, j = kJ ? kJ : a.j, nb = C + j, size = 1 << nb;
+    const int C = a.C, j = a.j, nb = C + j, size = 1 << nb;
     const int cmask = (1 << C) - 1;
     const int lane = threadIdx.x & 31;
     T *tp = reinterpret_cast<T *>(smem);
@@ -3605,11 +3600,11 @@ cudaError_t launch_block_bytes(const ChunkMeta *meta, const uint8_t *mask, uint3
     return cudaGetLastError();
 }
 
-template <typename R, int kC, int kJ>
-static cudaError_t launch_adjoint_pass_kc(const AdjPassArgs &a, cudaStream_t s) {
+template <typename R>
+static cudaError_t launch_adjoint_pass_any(const AdjPassArgs &a, cudaStream_t s) {
     const int nb = a.C + a.j;
     const size_t smem = (size_t)(4 * sizeof(R)) << nb;
-    auto kern = adjoint_pass_kernel<R, kC, kJ>;
+    auto kern = adjoint_pass_kernel<R>;
     cudaError_t e = ensure_dyn_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -3633,7 +3628,7 @@ static cudaError_t launch_adjoint_pass_t(const AdjPassArgs &a, const PassProgram
                           !a.rops || !a.pool))
         return cudaErrorInvalidValue;
     constexpr int kAC = 5, kAJ = sizeof(R) == 8 ? 6 : 7;
-    if (a.C != kAC || a.j != kAJ || !prog || a.nsweeps == 0) return launch_adjoint_pass_kc<R, 0, 0>(a, s);
+    if (a.C != kAC || a.j != kAJ || !prog || a.nsweeps == 0) return launch_adjoint_pass_any<R>(a, s);
     const size_t smem = 2 * tile_bytes<R>(kAC + kAJ);
     auto kern = adjoint_prog_kernel<R, kRB, kAC, kAJ>;
     cudaError_t e = ensure_dyn_smem(kern, smem);
