@@ -1705,10 +1705,15 @@ static bool plan_layout_passes(const std::vector<CGate> &sg, int n, int C, int j
     size_t left = G;
     // how soon a qubit is wanted again: its first unplaced gate, then the
     // chunk qubits of the final order
+    std::vector<std::vector<size_t>> mixers(n);
+    std::vector<size_t> next_mixer(n, 0);
+    for (size_t i = 0; i < G; ++i)
+        for (int q = 0; q < n; ++q)
+            if ((mix[i] >> q) & 1) mixers[q].push_back(i);
     auto wanted = [&](int q) -> size_t {
-        for (size_t i = 0; i < G; ++i)
-            if (!placed[i] && ((mix[i] >> q) & 1)) return i;
-        return q < C ? G : G + 1;
+        size_t &k = next_mixer[q];
+        while (k < mixers[q].size() && placed[mixers[q][k]]) ++k;
+        return k < mixers[q].size() ? mixers[q][k] : q < C ? G : G + 1;
     };
     while (left > 0 || (carried & low) != low) {
         if (steps.size() >= max_passes) return false;  // not better than the fixed order
