@@ -65,6 +65,11 @@ class ControlQubitInfo:
         return f"C({self.index},{self.value})"
 
 
+def keeps(cls, base, names) -> bool:
+    """Whether a gate class is base or takes the named methods from it."""
+    return issubclass(cls, base) and all(getattr(cls, name) is getattr(base, name) for name in names)
+
+
 class QuantumGateBase:
     """Base of every gate: name, qubit infos, matrix and property bits."""
 
@@ -98,7 +103,8 @@ class QuantumGateBase:
 
     def _matrix_entries(self) -> List[float]:
         """get_matrix() as interleaved doubles, row by row."""
-        m = self._matrix if type(self).get_matrix is QuantumGateBase.get_matrix else self.get_matrix()
+        plain = type(self).get_matrix is QuantumGateBase.get_matrix and "get_matrix" not in self.__dict__
+        m = self._matrix if plain else self.get_matrix()
         return np.ascontiguousarray(m, dtype=np.complex128).reshape(-1).view(np.float64).tolist()
 
     def get_property_value(self) -> int:
@@ -192,7 +198,7 @@ class ParametricRotationGate(QuantumGateBase):
         return _rotation_matrix(self._axis, self._angle)
 
     def _matrix_entries(self) -> List[float]:
-        if type(self).get_matrix is not ParametricRotationGate.get_matrix:
+        if type(self).get_matrix is not ParametricRotationGate.get_matrix or "get_matrix" in self.__dict__:
             return super()._matrix_entries()
         # the entries of _rotation_matrix without an array
         c, s = math.cos(self._angle / 2), math.sin(self._angle / 2)

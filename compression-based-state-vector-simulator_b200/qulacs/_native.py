@@ -211,23 +211,38 @@ def check(status: int, handle=None, dense: bool = False) -> None:
 def make_gate_array(gates, inverse: bool = False):
     """Pack qulacs gate objects into a qs_gate array (to_matrix_gate with the
     original name kept, as python/cppsim_wrapper.cpp:465-482 does); inverse:
-    each gate's conjugate transpose.  The fields are gathered in lists and
-    written column by column through a numpy view of the array: a circuit is
-    packed on every call of an uncompressed state (248 gates: 2.2 -> 0.5 ms)."""
+    each gate's conjugate transpose.  A gate is any object with the public
+    accessors (get_name, the index and value lists, get_matrix).  The fields
+    are gathered in lists and written column by column through a numpy view of
+    the array: a circuit is packed on every call of an uncompressed state
+    (248 rotations and CNOTs, on one CPU: 1.9 ms gate by gate, 1.1 ms so)."""
+    from ._gates import QuantumGateBase, keeps
     n = len(gates)
     arr = (qs_gate * max(1, n))()
     if not n:
         return arr
+    classes = {type(g) for g in gates}
+    plain = {cls for cls in classes if keeps(cls, QuantumGateBase, ("get_target_index_list", "get_control_index_list",
+                                                                    "get_control_value_list"))}
+    entries = {cls for cls in classes if hasattr(cls, "_matrix_entries")}
     names, nt, nc, targets, controls, values, flat = [], [], [], [], [], [], []
     pad = ([0, 0], [0], [])
     for i, g in enumerate(gates):
-        tg = [t.index for t in g.target_qubit_list]
-        cl = [c.index for c in g.control_qubit_list]
-        cv = [c.value for c in g.control_qubit_list]
+        cls = type(g)
+        if cls in plain and not ("get_target_index_list" in g.__dict__ or "get_control_index_list" in g.__dict__ or
+                                 "get_control_value_list" in g.__dict__):
+            tg = [t.index for t in g.target_qubit_list]
+            cl = [c.index for c in g.control_qubit_list]
+            cv = [c.value for c in g.control_qubit_list]
+        else:
+            tg = list(g.get_target_index_list())
+            cl = list(g.get_control_index_list())
+            cv = list(g.get_control_value_list())[:len(cl)]
         if len(tg) > 2 or len(cl) > 2:
             raise QompsimError(QS_ERR_UNSUPPORTED_GATE,
                                f"gate {i} ({g.get_name()}): only single- or two-qubit gates are implemented")
-        m = g._matrix_entries()
+        m = g._matrix_entries() if cls in entries else np.ascontiguousarray(
+            g.get_matrix(), dtype=np.complex128).reshape(-1).view(np.float64).tolist()
         if len(m) > 32:
             raise QompsimError(QS_ERR_UNSUPPORTED_GATE, f"gate {i} ({g.get_name()}): matrix larger than 4x4")
         names.append(g.get_name().encode()[:23])
@@ -235,7 +250,7 @@ def make_gate_array(gates, inverse: bool = False):
         nc.append(len(cl))
         targets.append(tg + pad[len(tg)])
         controls.append(cl + pad[len(cl)])
-        values.append(cv + pad[len(cl)])
+        values.append(cv + pad[len(cv)])
         flat.append(m)
     v = np.frombuffer(arr, dtype=np.dtype(qs_gate))
     v["name"] = np.array(names, dtype="S24").view("S1").reshape(n, 24)
