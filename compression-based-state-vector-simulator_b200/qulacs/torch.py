@@ -34,12 +34,22 @@ def _masks_arrays(xs, zs):
 
 
 def _inverse_gate_array(gates):
-    """The packed inverses of gates.  Every gate class of this package inverts
-    to its conjugate transpose (a rotation's entries at -theta are exactly
-    those), taken for all of them at once; a class with a get_inverse of its
-    own is asked."""
-    from ._gates import QuantumGateBase
-    if all(type(g).get_inverse is QuantumGateBase.get_inverse for g in gates):
+    """The packed inverses of gates: all conjugate transposes at once where
+    get_inverse() gives each gate just that by this package's own code (a gate
+    without an angle, or a rotation, whose entries at -theta are exactly
+    those).  Where a class or an object brings its own version of what
+    get_inverse calls, the gates are asked for their inverses."""
+    from ._gates import ParametricPauliRotationGate, ParametricRotationGate, QuantumGateBase, keeps
+
+    def daggers(cls):
+        if not keeps(cls, QuantumGateBase, ("get_inverse", "copy")):
+            return False
+        return not hasattr(cls, "set_parameter_value") or any(
+            keeps(cls, c, ("get_matrix", "set_parameter_value"))
+            for c in (ParametricRotationGate, ParametricPauliRotationGate))
+
+    called = frozenset(("get_inverse", "copy", "get_matrix", "set_parameter_value"))
+    if all(daggers(cls) for cls in {type(g) for g in gates}) and all(called.isdisjoint(g.__dict__) for g in gates):
         return _n.make_gate_array(gates, inverse=True)
     return _n.make_gate_array([g.get_inverse() for g in gates])
 

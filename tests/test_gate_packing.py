@@ -1,5 +1,5 @@
 """Packing of gate objects for the engine (qulacs._native.make_gate_array): any
-object with the public accessors is taken at its word."""
+object with the public accessors is taken at its word, inverses included."""
 import numpy as np
 import pytest
 
@@ -60,8 +60,29 @@ def own_matrix():
     return g
 
 
-CASES = [AccessorsOnly, relabelled, own_accessor, own_matrix, lambda: ParametricRotationGate("X", 0, 1.1),
-         lambda: G.CNOT(2, 0), lambda: G.SWAP(1, 3)]
+class Phased(ParametricRotationGate):
+    """exp(i theta) times the rotation: its inverse is not read off one matrix
+    alone but asked for."""
+
+    def get_matrix(self):
+        return np.exp(1j * self._angle) * super().get_matrix()
+
+
+class Shifted(ParametricRotationGate):
+    """Setting the angle adds a quarter turn, so get_inverse() is no dagger."""
+
+    def set_parameter_value(self, value):
+        super().set_parameter_value(value + np.pi / 2)
+
+
+class OwnInverse(QuantumGateMatrix):
+    def get_inverse(self):
+        return G.X(0)
+
+
+CASES = [AccessorsOnly, relabelled, own_accessor, own_matrix, lambda: Phased("Y", 2, 0.7), lambda: Shifted("Z", 1, 0.4),
+         lambda: OwnInverse([1], MATRIX), lambda: ParametricRotationGate("X", 0, 1.1), lambda: G.CNOT(2, 0),
+         lambda: G.SWAP(1, 3)]
 
 
 def check(rec, g):
@@ -79,3 +100,11 @@ def test_packed_gate_is_what_its_accessors_say(make):
     arr = _native.make_gate_array([G.H(0), make()])
     check(arr[0], G.H(0))
     check(arr[1], make())
+
+
+@pytest.mark.parametrize("make", CASES[3:])
+def test_packed_inverse_is_what_get_inverse_says(make):
+    from qulacs.torch import _inverse_gate_array
+    arr = _inverse_gate_array([make(), G.T(1)])
+    check(arr[0], make().get_inverse())
+    check(arr[1], G.T(1).get_inverse())
