@@ -252,13 +252,22 @@ def make_gate_array(gates, inverse: bool = False):
         controls.append(cl + pad[len(cl)])
         values.append(cv + pad[len(cv)])
         flat.append(m)
+
+    def words(column):
+        # as a uint32 field takes them: an index that no qubit has (a negative
+        # one, say) reaches the engine, which refuses it
+        try:
+            return np.array(column, dtype=np.uint32)
+        except OverflowError:
+            return np.array([[int(x) & 0xFFFFFFFF for x in row] for row in column], dtype=np.uint32)
+
     v = np.frombuffer(arr, dtype=np.dtype(qs_gate))
     v["name"] = np.array(names, dtype="S24").view("S1").reshape(n, 24)
     v["ntargets"] = nt
     v["ncontrols"] = nc
-    v["targets"][:, :2] = targets
-    v["controls"][:, :2] = controls
-    v["control_values"][:, :2] = values
+    v["targets"][:, :2] = words(targets)
+    v["controls"][:, :2] = words(controls)
+    v["control_values"][:, :2] = words(values)
     for size in {len(m) for m in flat}:
         rows = [i for i, m in enumerate(flat) if len(m) == size]
         m = np.array([flat[i] for i in rows], dtype=np.float64).view(np.complex128)

@@ -1,5 +1,7 @@
 """Packing of gate objects for the engine (qulacs._native.make_gate_array): any
 object with the public accessors is taken at its word, inverses included."""
+import ctypes as ct
+
 import numpy as np
 import pytest
 
@@ -108,3 +110,14 @@ def test_packed_inverse_is_what_get_inverse_says(make):
     arr = _inverse_gate_array([make(), G.T(1)])
     check(arr[0], make().get_inverse())
     check(arr[1], G.T(1).get_inverse())
+
+
+@pytest.mark.parametrize("index", [-1, 1 << 31, (1 << 32) - 1])
+def test_index_of_no_qubit_is_the_engines_to_refuse(index):
+    L = _native.load_library()
+    g = G.DenseMatrix(index, np.eye(2))
+    arr = _native.make_gate_array([G.H(0), g])
+    assert arr[1].targets[0] == index % (1 << 32)
+    ns = ct.c_size_t()
+    assert L.qs_plan_stages(arr, 2, 6, 4, 1, ct.byref(ns), None, None, None, None) == _native.QS_ERR_ARG
+    assert b"range" in L.qs_last_error(None)
