@@ -349,7 +349,10 @@ std::vector<qs::Sweep> plan_sweeps(const std::vector<qs::KGate> &kg, size_t g0, 
 // gate whose earlier gates it does not commute with are done and whose mixing
 // bits still fit RB register bits (the rule of plan_passes_dag, within a
 // pass).  Each sweep costs every amplitude a trip through shared memory.
-std::vector<size_t> sweep_order(const std::vector<qs::KGate> &kg, size_t g0, int RB) {
+// reads (when given): qubits that gate g0 + i depends on besides its own
+// without mixing them.
+std::vector<size_t> sweep_order(const std::vector<qs::KGate> &kg, size_t g0, int RB,
+                                const std::vector<uint64_t> *reads = nullptr) {
     const size_t G = kg.size() - g0;
     std::vector<std::vector<uint32_t>> succ(G);
     std::vector<int> indeg(G, 0);
@@ -370,6 +373,11 @@ std::vector<size_t> sweep_order(const std::vector<qs::KGate> &kg, size_t g0, int
                 } else {
                     users[q].push_back((uint32_t)i);
                 }
+            }
+            for (uint64_t m = reads ? (*reads)[i] : 0; m; m &= m - 1) {
+                const int q = __builtin_ctzll(m);
+                if (last_mix[q] >= 0) preds.push_back((uint32_t)last_mix[q]);
+                users[q].push_back((uint32_t)i);
             }
             std::sort(preds.begin(), preds.end());
             preds.erase(std::unique(preds.begin(), preds.end()), preds.end());
@@ -1019,9 +1027,12 @@ std::vector<PassPlan> plan_passes(const std::vector<uint32_t> &gate_ids, const s
 // takes, in index order and repeatedly, every ready gate whose mixing qubits
 // >= C still fit the tile and whose other qubits >= C fit the outer
 // selectors; a gate made ready by one taken in this pass may join it.  A
-// pass's gate list is a valid order of its gates.
+// pass's gate list is a valid order of its gates.  reads (when given): per
+// gate of cg, qubits that it depends on besides its own without mixing them
+// (they take no place in the tile or among the selectors).
 std::vector<PassPlan> plan_passes_dag(const std::vector<uint32_t> &gate_ids, const std::vector<CGate> &cg, int C,
-                                      int jmax, int jmin, int pad_lo, int pad_hi) {
+                                      int jmax, int jmin, int pad_lo, int pad_hi,
+                                      const std::vector<uint64_t> *reads = nullptr) {
     const size_t G = gate_ids.size();
     std::vector<std::vector<uint32_t>> succ(G);
     std::vector<int> indeg(G, 0);
@@ -1031,12 +1042,15 @@ std::vector<PassPlan> plan_passes_dag(const std::vector<uint32_t> &gate_ids, con
         for (size_t i = 0; i < G; ++i) {
             const CGate &g = cg[gate_ids[i]];
             std::vector<uint32_t> preds;
-            for (int b = 0; b < g.nq; ++b) {
-                const int q = g.q[b];
+            auto room = [&](int q) {
                 if ((int)last_mix.size() <= q) {
                     last_mix.resize(q + 1, -1);
                     users.resize(q + 1);
                 }
+            };
+            for (int b = 0; b < g.nq; ++b) {
+                const int q = g.q[b];
+                room(q);
                 if (last_mix[q] >= 0) preds.push_back((uint32_t)last_mix[q]);
                 if (g.mix[b]) {
                     preds.insert(preds.end(), users[q].begin(), users[q].end());
@@ -1045,6 +1059,12 @@ std::vector<PassPlan> plan_passes_dag(const std::vector<uint32_t> &gate_ids, con
                 } else {
                     users[q].push_back((uint32_t)i);
                 }
+            }
+            for (uint64_t m = reads ? (*reads)[gate_ids[i]] : 0; m; m &= m - 1) {
+                const int q = __builtin_ctzll(m);
+                room(q);
+                if (last_mix[q] >= 0) preds.push_back((uint32_t)last_mix[q]);
+                users[q].push_back((uint32_t)i);
             }
             std::sort(preds.begin(), preds.end());
             preds.erase(std::unique(preds.begin(), preds.end()), preds.end());
@@ -1123,6 +1143,22 @@ std::vector<PassPlan> plan_passes_dag(const std::vector<uint32_t> &gate_ids, con
     return out;
 }
 
+// The qubits that a parametric gate's generator reads (its Z factors) and the
+// gate does not act on: a gate that mixes one of them does not commute with
+// the derivative sum.
+uint64_t generator_reads(const CGate &g, uint64_t gen_z, int n) {
+    uint64_t covered = 0;
+    for (int b = 0; b < g.nq; ++b) covered |= 1ull << g.q[b];
+    return gen_z & ~covered & ((1ull << n) - 1);
+}
+std::vector<uint64_t> all_generator_reads(const std::vector<CGate> &cg, const int32_t *slots, const uint64_t *gen_z,
+                                          int n) {
+    std::vector<uint64_t> reads(cg.size(), 0);
+    for (size_t i = 0; i < cg.size(); ++i)
+        if (slots[i] >= 0) reads[i] = generator_reads(cg[i], gen_z[i], n);
+    return reads;
+}
+
 bool plan_dual_sweeps(const std::vector<CGate> &cg, const std::vector<uint32_t> &gl, const int32_t *slots,
                       const uint64_t *gen_x, const uint64_t *gen_z, const std::vector<int> &tile, int C, int RB,
                       std::vector<qs::Sweep> *all_sw, std::vector<qs::ROp> *all_rops, std::vector<cplx> *all_pool,
@@ -1132,22 +1168,26 @@ bool plan_dual_sweeps(const std::vector<CGate> &cg, const std::vector<uint32_t> 
     std::vector<qs::KGate> kg;
     std::vector<int32_t> sum_slot;
     std::vector<uint32_t> gid;
+    std::vector<uint64_t> reads;
     int32_t ls = 0;
     for (uint32_t gi : gl) {
         const qs::KGate g = to_kgate(cg[gi], tile, C);
         if (slots[gi] >= 0) {
             kg.push_back(g);
+            reads.push_back(generator_reads(cg[gi], gen_z[gi], 63));
             sum_slot.push_back(ls++);
             gid.push_back(gi);
         }
         kg.push_back(g);
+        reads.push_back(0);
         sum_slot.push_back(-1);
         gid.push_back(gi);
     }
     {
         // a sum keeps its place before every gate that does not commute with
-        // its generator: it carries its gate's qubits and mixing bits
-        const std::vector<size_t> order = sweep_order(kg, 0, RB);
+        // its generator: it carries its gate's qubits and mixing bits, and
+        // reads the qubits of the generator's other Z factors
+        const std::vector<size_t> order = sweep_order(kg, 0, RB, &reads);
         const auto kg0 = kg;
         const auto sum0 = sum_slot;
         const auto gid0 = gid;
@@ -3521,8 +3561,10 @@ qs_status qs_adjoint(qs_state *psi, qs_state *lam, const qs_gate *gates, const i
     // derivative sum of gate k commutes with U_k, so it shares with U_k only
     // qubits on which neither mixes, and there P_k is I or Z (its flip qubits
     // count as mixing qubits of gate k above); then G commutes with P_k and
-    // <G^-1 lam| P_k |G^-1 psi> = <lam| P_k |psi>.
-    auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, cg, C, jmax, jmax, C, n)
+    // <G^-1 lam| P_k |G^-1 psi> = <lam| P_k |psi>.  A Z factor of P_k on a
+    // qubit that gate k does not act on orders gate k like a use of that qubit.
+    const std::vector<uint64_t> reads = all_generator_reads(cg, slots, gen_z, n);
+    auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, cg, C, jmax, jmax, C, n, &reads)
                                              : plan_passes(ids, cg, C, jmax, jmax, C, n);
     // launches: a pass's gates, split so that each launch has at most
     // kMaxDualSlots derivative sums
@@ -4471,7 +4513,8 @@ qs_status qs_dense_adjoint(qs_dense *psi, qs_dense *lam, const qs_gate *gates, c
     std::vector<uint32_t> ids(count);
     for (size_t i = 0; i < count; ++i) ids[i] = (uint32_t)i;
     // commuting gates may change places (the argument at qs_adjoint holds here)
-    auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, cg, C, jmax, jmax, C, n)
+    const std::vector<uint64_t> reads = all_generator_reads(cg, slots, gen_z, n);
+    auto pl = env_int("QOMPSIM_DAG_PLAN", 1) ? plan_passes_dag(ids, cg, C, jmax, jmax, C, n, &reads)
                                              : plan_passes(ids, cg, C, jmax, jmax, C, n);
     // every launch's gate records (at most 128 parametric gates each) are
     // built first and uploaded at once; the launches then run back to back

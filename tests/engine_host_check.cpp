@@ -43,6 +43,10 @@
 //       register bits: its ops, interpreted by a host restatement of the
 //       two-store tile pass, give every derivative sum and both final states
 //       of the gates applied one by one
+//   engine_host_check dualreads
+//       the same with Z factors of the generators on qubits that their gates
+//       do not act on: no gate that mixes such a qubit changes sides with the
+//       sum, neither between passes nor inside one
 //   engine_host_check halfchains
 //       fuse_half_chains on random op lists of two sweeps: runs of
 //       half-diagonals on one register bit become pending factors (ACC) and
@@ -751,7 +755,7 @@ static void random_unitary(int dim, cplx *m, std::mt19937 &rng) {
 // ops, interpreted by host_dual_pass, give for each parametric gate
 // sum_x conj(B[x ^ gx]) (-1)^{|x & gz|} A[x] taken just before the gate,
 // and the states of every gate applied to both stores one by one.
-static int check_dualcompile() {
+static int check_dualcompile(bool reads_beyond) {
     std::mt19937 rng(19);
     std::uniform_real_distribution<double> u(-1.0, 1.0);
     const cplx one(1.0, 0.0), zero(0.0, 0.0);
@@ -785,6 +789,11 @@ static int check_dualcompile() {
                     if (pk == 2 || pk == 3) gz[k] |= 1ull << g.q[b];
                     if (pk == 1 || pk == 2) g.mix[b] = true;  // as qs_dense_adjoint: flipped qubits mix
                 }
+                if (reads_beyond)
+                    for (int z = 0; z < 2; ++z) {
+                        const int q = (int)(rng() % n);
+                        if (q != g.q[0] && (g.nq == 1 || q != g.q[1])) gz[k] |= 1ull << q;
+                    }
             }
             cg.push_back(g);
         }
@@ -803,7 +812,8 @@ static int check_dualcompile() {
         std::vector<cplx> ga(a0), gb(b0), got(nslot, 0.0);
         std::vector<uint32_t> ids(G);
         for (int k = 0; k < G; ++k) ids[k] = (uint32_t)k;
-        auto pl = plan_passes_dag(ids, cg, C, jmax, std::min(jmax, 3), C, n);
+        const std::vector<uint64_t> reads = all_generator_reads(cg, slots.data(), gz.data(), n);
+        auto pl = plan_passes_dag(ids, cg, C, jmax, std::min(jmax, 3), C, n, &reads);
         for (auto &pp : pl) {
             std::set<int> ts(pp.tile.begin(), pp.tile.end());
             for (int q = C; q < n && C + (int)ts.size() < RB; ++q) ts.insert(q);
@@ -857,7 +867,8 @@ static int check_dualcompile() {
                 return 1;
             }
     }
-    printf("dualcompile ok %ld of %ld passes fused, %ld sums\n", fused_passes, passes, nsum);
+    printf("%s ok %ld of %ld passes fused, %ld sums\n", reads_beyond ? "dualreads" : "dualcompile", fused_passes,
+           passes, nsum);
     return fused_passes > passes / 2 && nsum > 0 ? 0 : 1;
 }
 
@@ -926,7 +937,8 @@ int main(int argc, char **argv) {
     if (argc > 1 && !strcmp(argv[1], "selruns")) return check_selruns();
     if (argc > 1 && !strcmp(argv[1], "chunkperm")) return check_chunkperm();
     if (argc > 1 && !strcmp(argv[1], "opcompile")) return check_opcompile();
-    if (argc > 1 && !strcmp(argv[1], "dualcompile")) return check_dualcompile();
+    if (argc > 1 && !strcmp(argv[1], "dualcompile")) return check_dualcompile(false);
+    if (argc > 1 && !strcmp(argv[1], "dualreads")) return check_dualcompile(true);
     if (argc > 1 && !strcmp(argv[1], "dagplan")) return check_dagplan();
     if (argc > 1 && !strcmp(argv[1], "halfchains")) return check_halfchains();
     if (argc > 1 && !strcmp(argv[1], "headers")) return check_headers();

@@ -88,6 +88,13 @@ def test_two_store_op_compiler_sums_and_states(checker):
     assert r.returncode == 0 and "dualcompile ok" in r.stdout, r.stdout + r.stderr
 
 
+def test_generators_reading_other_qubits(checker):
+    """A generator may have Z factors on qubits that its gate does not act on:
+    the planners keep the gates that mix those on their side of the sum."""
+    r = subprocess.run([checker, "dualreads"], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "dualreads ok" in r.stdout, r.stdout + r.stderr
+
+
 def test_half_diagonal_chain_fusion(checker):
     """Runs of half-diagonals on one register bit fused into pending factors
     and one application give every register group the unfused result, and
