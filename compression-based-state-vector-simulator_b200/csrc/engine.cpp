@@ -1871,8 +1871,8 @@ struct HostPlan {
 // only becomes one header pass.  *last_gate (when given) receives, per pass,
 // the number k such that gates sg[0..k) have all been applied once the pass
 // is done (passes may take commuting gates out of order).  layout: every block
-// is stored, so the passes may change the order of the qubits as they go
-// (plan_layout_passes) when that takes fewer of them.
+// is stored and the arena has room, so the passes may change the order of the
+// qubits as they go (plan_layout_passes) when that takes fewer of them.
 static qs_status emit_passes(qs_state *h, uint32_t stage, const std::vector<CGate> &sg, const HostPerm &P,
                              HostPlan *plan, std::vector<qs_state::DevPass> *out, std::vector<size_t> *last_gate,
                              bool layout) {
@@ -2038,6 +2038,27 @@ static qs_status plan_device_passes(qs_state *h, HostPlan *plan) {
     return QS_OK;
 }
 
+// Whether the arena holds the state in whatever order of its qubits.  How well
+// a store packs depends on which amplitudes share a chunk, so a store between
+// two reordering passes can be larger than any in the register's order; in an
+// arena sized for the latter (n = 34, QOMPSIM_ARENA_BYTES) the fixed order
+// stays.  Bound: every chunk as wide as codes of both signs up to
+// |x| = 2^(L-m+1) make it (one bit more than amplitudes of a normalised state
+// need), plus what slabs of the default size leave unused: less than a chunk at
+// the end of each, and the last slab of each CTA (launch_pass: at most an
+// eighth of the arena).
+static bool arena_holds_any_order(const qs_state *h) {
+    const int64_t over = std::max<int64_t>(0, (int64_t)h->codec.L - h->codec.m + 1);
+    const int64_t code = std::max<int64_t>(1, over) << h->codec.m;   // of |x| = 1
+    const uint32_t width =
+        code > qs::kCodeLimit / 2 ? 32u : std::min<uint32_t>(32u, qs::bit_length((uint32_t)(2 * code)) + 1);
+    const uint64_t chunk = qs::payload_bytes((int)h->C, width);
+    const uint64_t share = qs::kArenaSlabBytes / 16;  // of a warp, at least
+    const uint64_t store = h->nchunks * (chunk + chunk * chunk / share);
+    const uint64_t unused = std::min<uint64_t>(h->capacity / 8, 1024 * qs::kArenaSlabBytes);
+    return store <= h->capacity - unused;
+}
+
 // The passes of stages [s0, end) planned as one gate sequence: once every
 // block is stored, no stage boundary changes the zero mask or the active
 // groups (every group is active, a stored block stays stored), so the
@@ -2073,7 +2094,7 @@ static qs_status plan_tail_passes(qs_state *h, uint32_t s0, HostPlan *plan, std:
         kept_before[i + 1] = sg.size();
     }
     std::vector<size_t> last_gate;
-    qs_status st = emit_passes(h, s0, sg, P, plan, passes, &last_gate, true);
+    qs_status st = emit_passes(h, s0, sg, P, plan, passes, &last_gate, arena_holds_any_order(h));
     if (st != QS_OK) return st;
     for (size_t k = 0; k < stage_end.size(); ++k) {
         const size_t kept = kept_before[stage_end[k]];  // relabelled gates up to this stage's end
@@ -2531,10 +2552,14 @@ qs_status qs_apply_circuit(qs_state *h) {
     if (errflag == 2)
         return fail(h, QS_ERR_TIMEOUT,
                     "a pass gave up waiting for its staged chunk payloads (bounded wait); the state is invalid");
-    if (errflag)
+    if (errflag) {
+        bool reordered = false;
+        for (size_t p = 0; p < ntail; ++p) reordered = reordered || h->tail_passes[p].shuffle;
         return fail(h, QS_ERR_CAPACITY,
                     "compressed store overflowed its arena (" + std::to_string(h->capacity) +
-                        " bytes); the state is invalid.  Set QOMPSIM_ARENA_BYTES larger.");
+                        " bytes); the state is invalid.  Set QOMPSIM_ARENA_BYTES larger" +
+                        (reordered ? ", or QOMPSIM_LAYOUT=0 for stores in the register's order only." : "."));
+    }
     if (tile_passes) h->arena_used = ctr[h->cur];
     // stages inside the merged tail: every block active; the stored total at
     // a stage's end is the store written by the tail pass that applied the

@@ -14,6 +14,9 @@
 //   engine_host_check tail <gates file> <n> <B> <I> <f64>
 //       per start stage: passes of the per-stage plan from there, passes of
 //       the merged tail, and the tail pass that ends each stage
+//   engine_host_check arena <gates file> <n> <B> <I> <f64> <arena bytes>
+//       the merged tail from stage 0 for an arena of that size: its passes
+//       and how many of them store their tile in another order
 //   engine_host_check selruns
 //       encode_selector_runs on random selector sets: where the selectors
 //       form at most two runs of consecutive bits, the variant computed from
@@ -136,7 +139,9 @@ static int check_plan(const char *path, uint32_t n, uint32_t B, uint32_t I, bool
 // Plans every stage and, for each start stage s0, the merged tail of stages
 // [s0, end): prints the per-stage passes from s0 on, the tail's passes and
 // the tail pass that ends each stage.
-static int check_tail(const char *path, uint32_t n, uint32_t B, uint32_t I, bool f64) {
+// With an arena of arena_bytes only the tail from stage 0 is planned, and the
+// passes that store their tile in another order are counted.
+static int check_tail(const char *path, uint32_t n, uint32_t B, uint32_t I, bool f64, uint64_t arena_bytes = 0) {
     FILE *f = fopen(path, "rb");
     if (!f) return 2;
     uint64_t cnt = 0;
@@ -163,6 +168,18 @@ static int check_tail(const char *path, uint32_t n, uint32_t B, uint32_t I, bool
     make_block_groups(&h);
     HostPlan plan;
     if (plan_device_passes(&h, &plan) != QS_OK) return 2;
+    if (arena_bytes) {
+        h.capacity = arena_bytes;
+        if (!qs::codec_params(f64, 1e-3, 1e-7, &h.codec)) return 2;
+        HostPlan tp;
+        std::vector<qs_state::DevPass> passes;
+        std::vector<int> ends;
+        if (plan_tail_passes(&h, 0, &tp, &passes, &ends) != QS_OK) return 2;
+        int shuffled = 0;
+        for (const auto &dp : passes) shuffled += dp.shuffle ? 1 : 0;
+        printf("arena merged %zu shuffled %d\n", passes.size(), shuffled);
+        return 0;
+    }
     for (uint32_t s0 = 0; s0 + 1 < h.stages.size(); ++s0) {
         size_t per_stage = 0;
         for (const auto &dp : h.passes) per_stage += dp.stage >= s0 ? 1 : 0;
@@ -945,6 +962,9 @@ int main(int argc, char **argv) {
     if (argc > 6 && !strcmp(argv[1], "plan"))
         return check_plan(argv[2], (uint32_t)atoi(argv[3]), (uint32_t)atoi(argv[4]), (uint32_t)atoi(argv[5]),
                           atoi(argv[6]) != 0);
+    if (argc > 7 && !strcmp(argv[1], "arena"))
+        return check_tail(argv[2], (uint32_t)atoi(argv[3]), (uint32_t)atoi(argv[4]), (uint32_t)atoi(argv[5]),
+                          atoi(argv[6]) != 0, strtoull(argv[7], nullptr, 10));
     if (argc > 6 && !strcmp(argv[1], "tail"))
         return check_tail(argv[2], (uint32_t)atoi(argv[3]), (uint32_t)atoi(argv[4]), (uint32_t)atoi(argv[5]),
                           atoi(argv[6]) != 0);

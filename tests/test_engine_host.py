@@ -179,3 +179,36 @@ def test_merged_tail_plan(checker, tmp_path, f64):
         assert all(b >= a for a, b in zip(t["ends"], t["ends"][1:]))
         assert t["ends"][-1] == t["merged"] - 1
     assert tails[2]["merged"] * 3 < tails[2]["per_stage"] * 2
+
+
+@pytest.mark.parametrize("f64", [True, False])
+def test_reordered_tail_needs_an_arena_for_any_order(checker, tmp_path, f64):
+    """Brickwork n=20: a tail that changes the order of the qubits takes fewer
+    passes, and is planned only where the arena holds the widest store that a
+    normalised state has in any order (eps_rel 1e-3, eps_abs 1e-7: codes of both
+    signs take 15 bits, and one more is left for larger states; 1 KiB a chunk)."""
+    import ctypes as ct
+    from qulacs import _native
+    from qulacs.circuit import QuantumCircuitOptimizer
+    from qompsim import circuits as C
+    n, B, I = 20, 12, 4
+    c = C.brickwork(n, 20, seed=0)
+    QuantumCircuitOptimizer(sv_block_size=B).optimize(c, block_size=2)
+    arr = _native.make_gate_array(c._gates)
+    path = tmp_path / "gates.bin"
+    with open(path, "wb") as f:
+        f.write(struct.pack("<Q", len(c._gates)))
+        f.write(ct.string_at(ct.addressof(arr), ct.sizeof(_native.qs_gate) * len(c._gates)))
+
+    def tail(arena):
+        r = subprocess.run([checker, "arena", str(path), str(n), str(B), str(I), "1" if f64 else "0", str(arena)],
+                           capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0 and r.stdout.startswith("arena merged"), r.stdout + r.stderr
+        t = r.stdout.split()
+        return int(t[2]), int(t[4])
+
+    widest = (1 << (n - 8)) * 1024
+    roomy, fixed = tail((8 << n)), tail(widest)
+    assert roomy[1] > 0 and fixed[1] == 0 and roomy[0] < fixed[0]
+    # slabs leave at most an eighth of the arena and a 16th of the store unused
+    assert tail(int(widest * 17 / 16 * 8 / 7) + 8)[1] > 0

@@ -73,3 +73,47 @@ def test_reordered_tail_matches_dense_and_fixed_order(monkeypatch, n, B, layers,
     # one quantisation a pass, each at most eps_rel |x| / 2 + eps_abs / 2 per
     # component: the relative errors of the passes add up at worst
     assert got["1"][0] <= (0.5e-3 + 0.5e-7 * 2 ** ((n + 1) / 2)) * got["1"][2]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["complex128", "complex64"])
+def test_arena_that_holds_the_fixed_order_is_enough(monkeypatch, dtype):
+    """A chain whose amplitudes differ in size with the upper qubits only, so
+    that chunks of the lower ones pack best: in arenas from too small to roomy,
+    wherever the fixed order runs, so does the default, with the same masks."""
+    import qulacs
+    from qulacs import _native
+    from qulacs.circuit import QuantumCircuitOptimizer
+    n, B = 16, 10
+    c = qulacs.QuantumCircuit(n)
+    for q in range(n):
+        c.add_H_gate(q) if q < 8 else c.add_RY_gate(q, 0.4)
+    for layer in range(9):
+        for q in range(n):
+            c.add_RX_gate(q, 1e-3 * (1 + q / n))
+        for a in range(layer % 2, n - 1, 2):
+            c.add_CZ_gate(a, a + 1)
+    QuantumCircuitOptimizer(sv_block_size=B).optimize(c, block_size=2)
+
+    def run(layout, arena):
+        monkeypatch.setenv("QOMPSIM_LAYOUT", layout)
+        monkeypatch.setenv("QOMPSIM_ARENA_BYTES", str(arena))
+        st = qulacs.CompressedQuantumState(n, B, dtype=dtype, eps_rel=1e-3, eps_abs=1e-7, flags=_native.QS_FLAG_QUIET)
+        st.partition_and_register_circuit(c, 4, 0)
+        try:
+            st.apply_circuit()
+        except _native.QompsimError as e:
+            assert e.status == _native.QS_ERR_CAPACITY
+            return None
+        return st.get_zero_mask().tolist(), sum(st.get_block_bytes())
+
+    final = run("0", 8 << n)[1]
+    fits = []
+    for percent in range(90, 131):
+        arena = final * percent // 100
+        fixed = run("0", arena)
+        fits.append(fixed is not None)
+        if fixed is not None:
+            got = run("1", arena)
+            assert got is not None and got[0] == fixed[0], percent
+    assert fits[-1] and not fits[0]
