@@ -50,7 +50,8 @@ def _dense(n, gates):
 def test_reordered_tail_matches_dense_and_fixed_order(monkeypatch, n, B, layers, dtype):
     """Brickwork (a chain: the reordering tail takes fewer passes): within the
     codec's error budget of a dense vector, same masks and stage count as the
-    fixed order, and no larger an error."""
+    fixed order, and an error no larger than the fixed order's but for the
+    scatter of 2^14 and more roundings (well under 5 % of their norm)."""
     import qulacs
     from qulacs import _native
     from qulacs.circuit import QuantumCircuitOptimizer
@@ -72,7 +73,9 @@ def test_reordered_tail_matches_dense_and_fixed_order(monkeypatch, n, B, layers,
     assert got["1"][1] == got["0"][1] and got["1"][3] == got["0"][3]
     # one quantisation a pass, each at most eps_rel |x| / 2 + eps_abs / 2 per
     # component: the relative errors of the passes add up at worst
-    assert got["1"][0] <= (0.5e-3 + 0.5e-7 * 2 ** ((n + 1) / 2)) * got["1"][2]
+    for env in ("0", "1"):
+        assert got[env][0] <= (0.5e-3 + 0.5e-7 * 2 ** ((n + 1) / 2)) * got[env][2]
+    assert got["1"][0] <= 1.05 * got["0"][0]
 
 
 @pytest.mark.gpu
