@@ -525,11 +525,16 @@ class CompressedQuantumState:
 
     # ---- accounting
     def get_max_SV_bytes(self) -> int:
+        """The largest entry of get_SV_bytes_history()."""
         v = _n.ct.c_uint64()
         self._check(_n.lib().qs_get_max_sv_bytes(self._h, _n.ct.byref(v)))
         return v.value
 
     def get_SV_bytes_history(self) -> List[int]:
+        """Stored bytes at the start and after each stage.  A stage that shares
+        its passes with others (once every block is stored) reports the store
+        written when its last gate had been applied, whose qubits may be in
+        another order than the register's; the last entry is the state."""
         cnt = _n.ct.c_size_t()
         self._check(_n.lib().qs_get_sv_bytes_history(self._h, None, 0, _n.ct.byref(cnt)))
         arr = (_n.ct.c_uint64 * max(1, cnt.value))()

@@ -315,11 +315,17 @@ qs_status qs_get_zero_mask(qs_state *h, uint8_t *out);
 qs_status qs_get_block_bytes(qs_state *h, uint64_t *out);
 
 /* get_max_SV_bytes() -- compressed_state.hpp:439-445: the largest total
- * over the initial state and every stage end. */
+ * over the initial state and every stage end (see qs_get_sv_bytes_history). */
 qs_status qs_get_max_sv_bytes(qs_state *h, uint64_t *out);
 
 /* Totals after the initial state and after each stage ("Total SV bytes",
- * compressed_state.hpp:374-437).  *count receives the number available. */
+ * compressed_state.hpp:374-437).  *count receives the number available.
+ * Stages that share passes (once every block is stored) report the store that
+ * was written when the stage's last gate had been applied.  That store may hold
+ * gates of later stages already, and its qubits may be in another order than
+ * the register's, in which it packs better or worse than the stage's own state
+ * would (QOMPSIM_LAYOUT=0 keeps the order, QOMPSIM_MERGE_TAIL=0 the stages).
+ * The last entry is always the stored state itself. */
 qs_status qs_get_sv_bytes_history(qs_state *h, uint64_t *out, size_t cap, size_t *count);
 
 /* get_total_times() -- python/cppsim_wrapper.cpp:503-515, the same ten keys

@@ -120,3 +120,32 @@ def test_arena_that_holds_the_fixed_order_is_enough(monkeypatch, dtype):
             got = run("1", arena)
             assert got is not None and got[0] == fixed[0], percent
     assert fits[-1] and not fits[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["complex128", "complex64"])
+def test_byte_totals_of_a_reordered_tail(monkeypatch, dtype):
+    """Every stage has a total in both orders; the last is the state's, the
+    same in both up to the codes that differ, and none passes the widest store
+    of a normalised state (16 bits a component and a 16-byte header a chunk)."""
+    import qulacs
+    from qulacs import _native
+    from qulacs.circuit import QuantumCircuitOptimizer
+    from qompsim import circuits as C
+    n, B = 17, 11
+    c = C.brickwork(n, 10, seed=n)
+    QuantumCircuitOptimizer(sv_block_size=B).optimize(c, block_size=2)
+    last = {}
+    for env in ("0", "1"):
+        monkeypatch.setenv("QOMPSIM_LAYOUT", env)
+        st = qulacs.CompressedQuantumState(n, B, dtype=dtype, eps_rel=1e-3, eps_abs=1e-7, flags=_native.QS_FLAG_QUIET)
+        st.partition_and_register_circuit(c, 4, 0)
+        st.apply_circuit()
+        history = st.get_SV_bytes_history()
+        assert len(history) == st.get_stats()["stages"] + 1
+        assert history[-1] == sum(int(b) for b in st.get_block_bytes())
+        assert st.get_max_SV_bytes() == max(history) <= (1 << (n - 8)) * (1024 + 16)
+        last[env] = history[-1]
+    # a chunk's width moves by a bit at most (its largest code by the passes'
+    # relative error, far below a factor of two), so its payload by one row
+    assert abs(last["1"] - last["0"]) <= (1 << (n - 8)) * 128
