@@ -9,6 +9,10 @@ with the kernel the reference would call for that gate:
 * a matrix gate without controls -> single_qubit_dense_matrix_gate or
   double_qubit_dense_matrix_gate_c (gate_matrix.cpp:128-160 dispatch)
 * with controls -> multi_qubit_control_multi_qubit_dense_matrix_gate
+
+Where that library is not built (the reference is not mounted), the same calls
+run this package's own plain statement of them (dense_oracle.cpp, in
+oracle/build/liboracle.so); available() tells which one checks.
 """
 from __future__ import annotations
 
@@ -28,34 +32,40 @@ def available() -> bool:
     return os.path.exists(LIB_PATH)
 
 
-def lib():
-    global _lib
-    if _lib is None:
-        if not available():
-            raise FileNotFoundError(f"{LIB_PATH} missing: run `make -C oracle` where the reference is mounted")
-        L = ct.CDLL(LIB_PATH)
+class _Kernels:
+    """The library's functions by their names without the prefix."""
+
+    def __init__(self, library, prefix):
         P = ct.c_void_p
         U = ct.c_uint
         U64 = ct.c_uint64
-        L.csimref_dense1.argtypes = [U, P, P, U64]
-        L.csimref_dense2.argtypes = [U, U, P, P, U64]
-        L.csimref_dense_multi.argtypes = [P, U, P, P, U64]
-        L.csimref_controlled.argtypes = [P, P, U, P, U, P, P, U64]
-        L.csimref_cnot.argtypes = [U, U, P, U64]
-        L.csimref_cz.argtypes = [U, U, P, U64]
-        L.csimref_swap.argtypes = [U, U, P, U64]
-        L.csimref_norm_squared.argtypes = [P, U64]
-        L.csimref_norm_squared.restype = ct.c_double
-        L.csimref_inner_product.argtypes = [P, P, U64, P]
-        L.csimref_init_zero.argtypes = [P, U64]
-        L.csimref_max_threads.restype = ct.c_int
-        _lib = L
+        for name, restype, argtypes in (
+                ("dense1", None, [U, P, P, U64]), ("dense2", None, [U, U, P, P, U64]),
+                ("dense_multi", None, [P, U, P, P, U64]), ("controlled", None, [P, P, U, P, U, P, P, U64]),
+                ("cnot", None, [U, U, P, U64]), ("cz", None, [U, U, P, U64]), ("swap", None, [U, U, P, U64]),
+                ("norm_squared", ct.c_double, [P, U64]), ("inner_product", None, [P, P, U64, P]),
+                ("init_zero", None, [P, U64]), ("max_threads", ct.c_int, [])):
+            f = getattr(library, prefix + name)
+            f.restype, f.argtypes = restype, argtypes
+            setattr(self, name, f)
+
+
+def dense_kernels() -> _Kernels:
+    """dense_oracle.cpp's functions."""
+    from . import codec
+    return _Kernels(codec.lib(), "qsor_dense_")
+
+
+def lib() -> _Kernels:
+    global _lib
+    if _lib is None:
+        _lib = _Kernels(ct.CDLL(LIB_PATH), "csimref_") if available() else dense_kernels()
     return _lib
 
 
 def zero_state(n: int) -> np.ndarray:
     s = np.empty(1 << n, dtype=np.complex128)
-    lib().csimref_init_zero(s.ctypes.data, s.size)
+    lib().init_zero(s.ctypes.data, s.size)
     return s
 
 
@@ -72,28 +82,28 @@ def apply_gate(state: np.ndarray, g) -> None:
     c = g.get_control_index_list()
     cv = g.get_control_value_list()
     if name == "CNOT":
-        L.csimref_cnot(c[0], t[0], _ptr(state), dim)
+        L.cnot(c[0], t[0], _ptr(state), dim)
         return
     if name == "CZ":
-        L.csimref_cz(c[0], t[0], _ptr(state), dim)
+        L.cz(c[0], t[0], _ptr(state), dim)
         return
     if name == "SWAP":
-        L.csimref_swap(t[0], t[1], _ptr(state), dim)
+        L.swap(t[0], t[1], _ptr(state), dim)
         return
     m = np.ascontiguousarray(g.get_matrix(), dtype=np.complex128)
     if not c:
         if len(t) == 1:
-            L.csimref_dense1(t[0], _ptr(m), _ptr(state), dim)
+            L.dense1(t[0], _ptr(m), _ptr(state), dim)
         elif len(t) == 2:
-            L.csimref_dense2(t[0], t[1], _ptr(m), _ptr(state), dim)
+            L.dense2(t[0], t[1], _ptr(m), _ptr(state), dim)
         else:
             ta = np.asarray(t, dtype=np.uint32)
-            L.csimref_dense_multi(_ptr(ta), len(t), _ptr(m), _ptr(state), dim)
+            L.dense_multi(_ptr(ta), len(t), _ptr(m), _ptr(state), dim)
         return
     ca = np.asarray(c, dtype=np.uint32)
     va = np.asarray(cv, dtype=np.uint32)
     ta = np.asarray(t, dtype=np.uint32)
-    L.csimref_controlled(_ptr(ca), _ptr(va), len(c), _ptr(ta), len(t), _ptr(m), _ptr(state), dim)
+    L.controlled(_ptr(ca), _ptr(va), len(c), _ptr(ta), len(t), _ptr(m), _ptr(state), dim)
 
 
 def apply_gates(state: np.ndarray, gates: Sequence) -> np.ndarray:
@@ -108,14 +118,14 @@ def run_circuit(n: int, gates: Sequence, init: np.ndarray | None = None) -> np.n
 
 
 def norm_squared(state: np.ndarray) -> float:
-    return float(lib().csimref_norm_squared(_ptr(state), state.size))
+    return float(lib().norm_squared(_ptr(state), state.size))
 
 
 def inner_product(bra: np.ndarray, ket: np.ndarray) -> complex:
     out = np.zeros(2)
-    lib().csimref_inner_product(_ptr(bra), _ptr(ket), bra.size, _ptr(out))
+    lib().inner_product(_ptr(bra), _ptr(ket), bra.size, _ptr(out))
     return complex(out[0], out[1])
 
 
 def max_threads() -> int:
-    return int(lib().csimref_max_threads())
+    return int(lib().max_threads())
