@@ -101,12 +101,6 @@ class QuantumGateBase:
     def get_matrix(self) -> np.ndarray:
         return self._matrix.copy()
 
-    def _matrix_entries(self) -> List[float]:
-        """get_matrix() as interleaved doubles, row by row."""
-        plain = type(self).get_matrix is QuantumGateBase.get_matrix and "get_matrix" not in self.__dict__
-        m = self._matrix if plain else self.get_matrix()
-        return np.ascontiguousarray(m, dtype=np.complex128).reshape(-1).view(np.float64).tolist()
-
     def get_property_value(self) -> int:
         return self._gate_property
 
@@ -197,9 +191,8 @@ class ParametricRotationGate(QuantumGateBase):
     def get_matrix(self) -> np.ndarray:
         return _rotation_matrix(self._axis, self._angle)
 
-    def _matrix_entries(self) -> List[float]:
-        if type(self).get_matrix is not ParametricRotationGate.get_matrix or "get_matrix" in self.__dict__:
-            return super()._matrix_entries()
+    def _entries(self) -> List[float]:
+        """get_matrix() as interleaved doubles, row by row."""
         # the entries of _rotation_matrix without an array
         c, s = math.cos(self._angle / 2), math.sin(self._angle / 2)
         if self._axis == "X":
