@@ -236,8 +236,9 @@ __host__ __device__ inline float f32_from(uint32_t b) {
 // The signed forms below fold the sign into the linear region's rounding
 // constant (1.5 * 2^52, 1.5 * 2^23: rint is symmetric, so rint(x 2^L) is
 // +-rint(|x| 2^L) and its two's complement appears in the low word / bits),
-// and the log region's two additions into one constant: 9 instead of 13
-// instructions a component to quantise, 7 instead of 11 to dequantise.
+// and the log region's two additions into one constant: by the operations
+// written here, 9 instead of 13 a component to quantise, 7 instead of 11 to
+// dequantise.
 //
 // m <= kFastMantissaF64.  The log region needs no clamp: its shift is at
 // least 1, so the code is at most (2^31 - 1) >> 1 = kCodeLimit.

@@ -1499,12 +1499,13 @@ qs_status qs_create(qs_state **out, uint32_t n, uint32_t block_size, qs_dtype dt
     if (env_int("QOMPSIM_HOST_STORE", 0)) flags |= QS_FLAG_HOST_STORE;
     h->flags = flags;
     h->host_store = (flags & QS_FLAG_HOST_STORE) != 0;
-    // Tile passes run pass_kernel (three 4-warp CTAs per SM, payloads copied
-    // chunk by chunk with cp.async) unless QOMPSIM_STAGED_PASS=1 selects
-    // staged_pass_kernel (payloads of the next tile prefetched with bulk
-    // copies), which measured 1.3-1.8x slower per pass on the QFT: its
-    // registers leave one 8-warp CTA per SM, and the passes are bound by
-    // the latency of their decode / sweep / quantise phases, not by memory.
+    // Tile passes run pass_kernel (PassShape: two or three CTAs an SM, every
+    // payload copy of a warp's chunks started at once) unless
+    // QOMPSIM_STAGED_PASS=1 selects staged_pass_kernel (payloads of the next
+    // tile prefetched with bulk copies), which is slower: QFT n=29 complex128
+    // 85.5 against 59.7 ms, complex64 77.9 against 40.0 ms.  Its buffers leave
+    // one CTA per SM (kStagedThreads), it reads its ops from global memory, and
+    // the passes are bound by instruction issue and latency, not by memory.
     // Dense k-qubit passes always use the staged kernel (it holds the tensor
     // core operands); so that they can run, the host-store arenas (read with
     // cp.async) are excluded from it.
@@ -1675,8 +1676,6 @@ static void make_block_groups(qs_state *h) {
     }
 }
 
-// The device passes of every stage as host data: h->passes plus the op
-// records, sweeps and matrix pool they index.  Host code only.
 // Passes that change the order of the qubits as they go.  A chunk fixes its C
 // lowest qubits, so a tile holds those and jmax others, and a pass that starts
 // from the register's own order spends C of its tile on qubits 0..C-1 whether or
@@ -1858,6 +1857,8 @@ static bool plan_layout_passes(const std::vector<CGate> &sg, int n, int C, int j
     return true;
 }
 
+// The device passes of every stage as host data: h->passes plus the op
+// records, sweeps and matrix pool they index.  Host code only.
 struct HostPlan {
     std::vector<qs::KGate> kg;
     std::vector<qs::Sweep> sw;

@@ -3272,10 +3272,12 @@ static cudaError_t launch_pass_kc(const PassArgs &a, const Prog &prog, cudaStrea
 // The default chunk size (2^8 amplitudes) and the default tile (2^12
 // amplitudes for complex128, 2^13 for complex64, i.e. 4 or 5 tile qubits
 // above the chunk) are compile-time constants of their instantiation: the
-// per-lane counts, chunk and group counts, offsets and swizzle mask then fold
-// into the code (measured 12-19 % faster than reading them from the args).
+// per-lane counts, chunk and group counts and tile offsets then fold into the
+// code (12-19 % faster than reading them from the args, an earlier build).
 // These instantiations read their ops from a program; longer op lists run from
-// global memory in the run-time geometry.
+// global memory in the run-time geometry: n=25 complex128, dense two-qubit gates
+// on 12 qubits, 28 gates (the longest program) 2.35 ms, 40 gates 3.65 ms, 300
+// gates 20.2 ms (the build before programs: 3.11, 3.88 and 21.2 ms).
 template <typename R, int RB, bool kCodes>
 static cudaError_t launch_pass_t(const PassArgs &a, const PassProgram *prog, cudaStream_t s) {
     constexpr int J = sizeof(R) == 8 ? 4 : 5;
