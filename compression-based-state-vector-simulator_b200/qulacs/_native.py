@@ -230,11 +230,15 @@ def make_gate_array(gates, inverse: bool = False):
             "get_matrix", "_entries"))
         known[cls] = keeps(cls, QuantumGateBase, lists), kind
     asked = frozenset(lists + ("get_matrix",))
+    try:
+        clean = all(map(asked.isdisjoint, map(vars, gates)))
+    except TypeError:  # an object without a __dict__
+        clean = False
     names, nt, nc, targets, controls, values, groups = [], [], [], [], [], [], {}
     pad = ([0, 0], [0], [])
     for i, g in enumerate(gates):
         plain, kind = known[type(g)]
-        if (plain or kind) and not asked.isdisjoint(g.__dict__):
+        if not clean and (plain or kind) and not asked.isdisjoint(vars(g)):
             plain = kind = 0  # the object itself brings accessors
         if plain:
             tg = [t.index for t in g.target_qubit_list]

@@ -49,7 +49,7 @@ def _inverse_gate_array(gates):
             for c in (ParametricRotationGate, ParametricPauliRotationGate))
 
     called = frozenset(("get_inverse", "copy", "get_matrix", "set_parameter_value"))
-    if all(daggers(cls) for cls in {type(g) for g in gates}) and all(called.isdisjoint(g.__dict__) for g in gates):
+    if all(daggers(cls) for cls in {type(g) for g in gates}) and all(map(called.isdisjoint, map(vars, gates))):
         return _n.make_gate_array(gates, inverse=True)
     return _n.make_gate_array([g.get_inverse() for g in gates])
 
