@@ -1,4 +1,4 @@
-"""The checker that stands in where the reference's csim kernels are not built
+"""The oracle that stands in where the reference's csim kernels are not built
 (oracle/dense_oracle.cpp), against the golden states that csim wrote, full
 matrix products and csim itself where it is there (CPU only)."""
 import numpy as np
